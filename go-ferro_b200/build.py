@@ -3,10 +3,9 @@
     python go-ferro_b200/build.py
 
 Two CUDA translation units: gf_engine.cu (the FP64 parity kernels, the host
-engine and the C ABI) is compiled with -fmad=false, so that every multiply
-and add is rounded as in the reference's host build; gf_mixed.cu (the FP32
-mixed-form stage kernels) is compiled with FMA contraction.  The library
-links cuFFT for the magnetostatic transforms.
+engine and the C ABI) and gf_mixed.cu (the FP32 mixed-form stage kernels),
+both compiled with FMA contraction.  The library links cuFFT for the
+magnetostatic transforms.
 """
 from __future__ import annotations
 
@@ -21,9 +20,9 @@ CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "libgoferro_b200.so")
 
 # (source, extra flags): each compiled to its own object, then linked
-UNITS = [("gf_engine.cu", ["-fmad=false"]), ("gf_mixed.cu", ["-fmad=true"]), ("gf_deck.cpp", [])]
+UNITS = [("gf_engine.cu", ["-fmad=true"]), ("gf_mixed.cu", ["-fmad=true"]), ("gf_deck.cpp", [])]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-O2", "-I" + os.path.join(ROOT, "include")]
+FLAGS = ["-O3", "-split-compile=4", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-O2", "-I" + os.path.join(ROOT, "include")]
 
 
 def nvcc() -> str:

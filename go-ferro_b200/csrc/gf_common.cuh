@@ -5,9 +5,10 @@
 // one byte per cell (0 = vacuum, id-1 indexes the material table), in place
 // of the reference's unsigned int material_cell (global.h:92).
 //
-// The FP64 parity kernels are compiled with -fmad=false and evaluate every
-// expression in the reference's operation order, so that each multiply and
-// add is rounded exactly as in the reference's host build.
+// The FP64 kernels follow the reference's operation order; the compiler may
+// contract a multiply and an add into one rounding, and divisions by run
+// constants are multiplications by the rounded reciprocal (qdivR).  Both agree
+// with the reference's host build to rounding (every golden trace to 1e-10).
 #pragma once
 
 #include <cstdint>
@@ -172,10 +173,14 @@ __device__ __forceinline__ double qdiv(double x, double d, double rd) {
     return x == 0. ? q0 : q2;
 }
 
-// Division by a run constant d: qdiv in the FP64 form (rd = RN(1/d)); in the
-// mixed form a multiplication by the FP32 reciprocal rdf (within one ulp of
-// the FP32 quotient).
-__device__ __forceinline__ double qdivR(double x, double d, double rd, float) { return qdiv(x, d, rd); }
+// Division by a run constant d in the stencils: a multiplication by its
+// rounded reciprocal (rd = RN(1/d), rdf in FP32), within one ulp of the
+// quotient.  qdiv's exact quotient costs five FP64 operations and a select
+// where this costs one, at up to 60 divisions per cell and stage (128^3
+// ferroelectric, FP64, us per launch with both this and contraction: elastic
+// tile 255 -> 230, Yee 152 -> 144, TDGL 134 -> 130); the LLG kernels' RK
+// weights keep qdiv.
+__device__ __forceinline__ double qdivR(double x, double, double rd, float) { return x * rd; }
 __device__ __forceinline__ float qdivR(float x, double, double, float rdf) { return x * rdf; }
 
 // frame-rotation matrices in the kernel's precision

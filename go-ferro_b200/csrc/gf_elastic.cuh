@@ -966,17 +966,17 @@ __device__ __forceinline__ void elastic_rk_body(const Params& P, const StageIOT<
         for (int a = 0; a < 3; a++) {
             const double du = vin[a] * P.dt;
             if (S == 0) {
-                io.v_out.c[a][c] = vx[a] + dv[a] * 0.5; io.v_acc.c[a][c] = vx[a] + qdiv(dv[a], 6., kInv6);
-                uo[a] = ux[a] + du * 0.5;               io.u_acc.c[a][c] = ux[a] + qdiv(du, 6., kInv6);
+                io.v_out.c[a][c] = vx[a] + dv[a] * 0.5; io.v_acc.c[a][c] = vx[a] + dv[a] * kInv6;
+                uo[a] = ux[a] + du * 0.5;               io.u_acc.c[a][c] = ux[a] + du * kInv6;
             } else if (S == 1) {
-                io.v_out.c[a][c] = vx[a] + dv[a] * 0.5; io.v_acc.c[a][c] = va[a] + qdiv(dv[a], 3., kInv3);
-                uo[a] = ux[a] + du * 0.5;               io.u_acc.c[a][c] = ua[a] + qdiv(du, 3., kInv3);
+                io.v_out.c[a][c] = vx[a] + dv[a] * 0.5; io.v_acc.c[a][c] = va[a] + dv[a] * kInv3;
+                uo[a] = ux[a] + du * 0.5;               io.u_acc.c[a][c] = ua[a] + du * kInv3;
             } else if (S == 2) {
-                io.v_out.c[a][c] = vx[a] + dv[a];       io.v_acc.c[a][c] = va[a] + qdiv(dv[a], 3., kInv3);
-                uo[a] = ux[a] + du;                     io.u_acc.c[a][c] = ua[a] + qdiv(du, 3., kInv3);
+                io.v_out.c[a][c] = vx[a] + dv[a];       io.v_acc.c[a][c] = va[a] + dv[a] * kInv3;
+                uo[a] = ux[a] + du;                     io.u_acc.c[a][c] = ua[a] + du * kInv3;
             } else {
-                io.v_acc.c[a][c] = va[a] + qdiv(dv[a], 6., kInv6);
-                uo[a] = ua[a] + qdiv(du, 6., kInv6);
+                io.v_acc.c[a][c] = va[a] + dv[a] * kInv6;
+                uo[a] = ua[a] + du * kInv6;
             }
         }
         const bool skip = P.el_bc_fused ? rk_bc_fused<S, double>(P, io, c, ux, uo, ucn) : false;

@@ -185,10 +185,10 @@ __device__ inline void rk_x(const YeeIn<R>& L, R d, R* out, R* acc, R* cmp, int 
             cmp[e] = err;
         }
     } else {
-        if (S == 0) { out[e] = xv + d * 0.5; acc[e] = xv + qdiv(d, 6., kInv6); }
-        else if (S == 1) { out[e] = xv + d * 0.5; acc[e] = L.acc + qdiv(d, 3., kInv3); }
-        else if (S == 2) { out[e] = xv + d; acc[e] = L.acc + qdiv(d, 3., kInv3); }
-        else { acc[e] = L.acc + qdiv(d, 6., kInv6); }
+        if (S == 0) { out[e] = xv + d * 0.5; acc[e] = xv + d * kInv6; }
+        else if (S == 1) { out[e] = xv + d * 0.5; acc[e] = L.acc + d * kInv3; }
+        else if (S == 2) { out[e] = xv + d; acc[e] = L.acc + d * kInv3; }
+        else { acc[e] = L.acc + d * kInv6; }
     }
 }
 
@@ -270,7 +270,7 @@ __device__ inline void em_E_edge(const Params& P, const StageIOT<R>& io, const S
             if constexpr (is_mixed<R>::value)
                 dP = dP * (pc == 3.f ? 1.f / 3.f : (pc == 1.f ? 1.f : (pc == 2.f ? 0.5f : 0.25f)));
             else
-                dP = qdiv(dP, pc, pc == 3. ? kInv3 : (pc == 1. ? 1. : (pc == 2. ? 0.5 : 0.25)));
+                dP = dP * (pc == 3. ? kInv3 : (pc == 1. ? 1. : (pc == 2. ? 0.5 : 0.25)));
             rhs = rhs - qdivR(dP, P.dt, P.rdt, P.f.rdt);
         }
         d = coef * rhs;
@@ -463,10 +463,10 @@ __global__ void __launch_bounds__(256) k_drude(Params P, StageIOT<R> io) {
                 double* out = io.jp_out[pole].c[a];
                 double* acc = io.jp_acc[pole].c[a];
                 const double xv = io.jp_x[pole].c[a][c];
-                if (S == 0) { out[c] = xv + d * 0.5; acc[c] = xv + qdiv(d, 6., kInv6); }
-                else if (S == 1) { out[c] = xv + d * 0.5; acc[c] = acc[c] + qdiv(d, 3., kInv3); }
-                else if (S == 2) { out[c] = xv + d; acc[c] = acc[c] + qdiv(d, 3., kInv3); }
-                else { acc[c] = acc[c] + qdiv(d, 6., kInv6); }
+                if (S == 0) { out[c] = xv + d * 0.5; acc[c] = xv + d * kInv6; }
+                else if (S == 1) { out[c] = xv + d * 0.5; acc[c] = acc[c] + d * kInv3; }
+                else if (S == 2) { out[c] = xv + d; acc[c] = acc[c] + d * kInv3; }
+                else { acc[c] = acc[c] + d * kInv6; }
             }
     }
 }

@@ -1,9 +1,8 @@
 // B200 engine for GO-Ferro's coupled RK4 phase-field step: state ownership,
 // stage sequencing, CUDA-graph replay and the C ABI of goferro_b200.h.
 //
-// One translation unit holds every kernel (the .cuh files below); it is
-// compiled with -fmad=false so that each multiply and add of the FP64 parity
-// form is rounded separately, as in the reference's host build.
+// One translation unit holds every FP64 kernel (the .cuh files below),
+// another (gf_mixed.cu) the FP32 stage kernels.
 //
 // Two precisions share the engine.  The FP64 form (GF_PRECISION_FP64) is the
 // parity path.  The mixed form (GF_PRECISION_MIXED_FP32) instantiates the

@@ -409,17 +409,17 @@ __device__ __forceinline__ void fe_rk(const Params& P, const StageIOT<R>& io, in
         for (int a = 0; a < 3; a++) {
             const double dp = qin[a] * P.dt;
             if (S == 0) {
-                io.q_out.c[a][c] = qx[a] + dq[a] * 0.5; io.q_acc.c[a][c] = qx[a] + qdiv(dq[a], 6., kInv6);
-                io.p_out.c[a][c] = px0[a] + dp * 0.5;   io.p_acc.c[a][c] = px0[a] + qdiv(dp, 6., kInv6);
+                io.q_out.c[a][c] = qx[a] + dq[a] * 0.5; io.q_acc.c[a][c] = qx[a] + dq[a] * kInv6;
+                io.p_out.c[a][c] = px0[a] + dp * 0.5;   io.p_acc.c[a][c] = px0[a] + dp * kInv6;
             } else if (S == 1) {
-                io.q_out.c[a][c] = qx[a] + dq[a] * 0.5; io.q_acc.c[a][c] = qa[a] + qdiv(dq[a], 3., kInv3);
-                io.p_out.c[a][c] = px0[a] + dp * 0.5;   io.p_acc.c[a][c] = pa[a] + qdiv(dp, 3., kInv3);
+                io.q_out.c[a][c] = qx[a] + dq[a] * 0.5; io.q_acc.c[a][c] = qa[a] + dq[a] * kInv3;
+                io.p_out.c[a][c] = px0[a] + dp * 0.5;   io.p_acc.c[a][c] = pa[a] + dp * kInv3;
             } else if (S == 2) {
-                io.q_out.c[a][c] = qx[a] + dq[a];       io.q_acc.c[a][c] = qa[a] + qdiv(dq[a], 3., kInv3);
-                io.p_out.c[a][c] = px0[a] + dp;         io.p_acc.c[a][c] = pa[a] + qdiv(dp, 3., kInv3);
+                io.q_out.c[a][c] = qx[a] + dq[a];       io.q_acc.c[a][c] = qa[a] + dq[a] * kInv3;
+                io.p_out.c[a][c] = px0[a] + dp;         io.p_acc.c[a][c] = pa[a] + dp * kInv3;
             } else {
-                io.q_acc.c[a][c] = qa[a] + qdiv(dq[a], 6., kInv6);
-                io.p_acc.c[a][c] = pa[a] + qdiv(dp, 6., kInv6);
+                io.q_acc.c[a][c] = qa[a] + dq[a] * kInv6;
+                io.p_acc.c[a][c] = pa[a] + dp * kInv6;
             }
         }
     }
