@@ -22,7 +22,7 @@ OUT = os.path.join(HERE, "libgoferro_b200.so")
 # (source, extra flags): each compiled to its own object, then linked
 UNITS = [("gf_engine.cu", ["-fmad=true"]), ("gf_mixed.cu", ["-fmad=true"]), ("gf_deck.cpp", [])]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-FLAGS = ["-O3", "-split-compile=4", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-O2", "-I" + os.path.join(ROOT, "include")]
+FLAGS = ["-O3", "-split-compile=8", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-O2", "-I" + os.path.join(ROOT, "include")]
 
 
 def nvcc() -> str:

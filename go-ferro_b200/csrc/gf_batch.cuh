@@ -39,6 +39,8 @@ struct BatchInst {
     StageIOT<float> io[2][4];          // [step parity][stage]
     const EmCls<float>* cls;
     int ncls, nmat, el_chunk, el_cubic;
+    int uni;                           // every cell is ferroelectric material 1, um
+    DevMatT<float> um;
     unsigned long long* step;          // the engine's step counter
 };
 
@@ -46,6 +48,13 @@ struct BatchInst {
 struct BatchItem {
     int inst, kind, bx, by, bz;
 };
+
+// the TDGL update of an item, in the form the engine alone uses
+template <int S>
+__device__ __forceinline__ void batch_fe(const BatchInst& g, const StageIOT<float>& io, const BatchItem it) {
+    if (g.uni) fe_body<S, float, false, true>(g.P, io, g.um, it.bx, it.by);
+    else fe_body<S, float, false, false>(g.P, io, g.um, it.bx, it.by);
+}
 
 // PH: 0 = phase A (all of its kinds), 1 = the later phases (RK update, Mur
 // and elastic boundaries), 3 = phase A tile items only, 4 = phase A Yee
@@ -73,13 +82,13 @@ __device__ __forceinline__ void batch_item(const BatchInst* __restrict__ insts, 
     if constexpr (PH == 0) {
         if (it.kind == BK_TILE) tile();
         else if (it.kind == BK_EM) yee();
-        else if (it.kind == BK_FE) fe_body<S, float, false>(P, io, it.bx, it.by);
+        else if (it.kind == BK_FE) batch_fe<S>(g, io, it);
     } else if constexpr (PH == 3) {
         tile();
     } else if constexpr (PH == 4) {
         yee();
     } else if constexpr (PH == 5) {
-        fe_body<S, float, false>(P, io, it.bx, it.by);
+        batch_fe<S>(g, io, it);
     } else {
         if (it.kind == BK_RK) elastic_rk_body<S, float>(P, io, it.bx);
         else if (it.kind == BK_MUR_X) em_mur_body<S, 0, float>(P, io, it.bx);
@@ -152,7 +161,7 @@ __device__ __noinline__ void batch_kind_call(const BatchInst* __restrict__ insts
         EmCls<float>* cl = reinterpret_cast<EmCls<float>*>(smem_raw + kMaxMat * sizeof(EmMat<float>));
         em_fused_body<S, float>(P, io, g.nmat, g.cls, g.ncls, it.bx, it.by, mt, cl);
     } else if constexpr (K == BK_FE) {
-        fe_body<S, float, false>(P, io, it.bx, it.by);
+        batch_fe<S>(g, io, it);
     } else if constexpr (K == BK_RK) {
         elastic_rk_body<S, float>(P, io, it.bx);
     } else if constexpr (K == BK_MUR_X) {

@@ -7,8 +7,7 @@
 //                 (get_eigenstrain_dynamic, :3-104), the six face stresses and
 //                 the stress divergence (the stress part of get_dv_RK{1..4}
 //                 :841-2800); it also stores the crystal-frame cell strain of
-//                 magnetic cells for the LLG kernels and, in the FP64 form, of
-//                 ferroelectric cells for the TDGL kernel.
+//                 magnetic cells for the LLG kernels.
 //   k_elastic_rk  per cell: damping terms, f_store, the velocity and
 //                 displacement increments and their RK4 combination
 //                 (get_dv_RK* :1295-1329, get_du_RK* :2801-2847,
@@ -105,13 +104,15 @@ template <class R, class M>
 __device__ inline void eigen_terms(const Params& P, const StageIOT<R>& io, long c, const M& mt, R mx, R my,
                                    R mz, R px, R py, R pz, const R e0[6], R e[6]) {
     const R third = R(1.) / R(3.);
-    R t[6];
-    t[0] = mt.l100_15 * (mx * mx - third);
-    t[1] = mt.l100_15 * (my * my - third);
-    t[2] = mt.l100_15 * (mz * mz - third);
-    t[3] = mt.l111_15 * my * mz;
-    t[4] = mt.l111_15 * mx * mz;
-    t[5] = mt.l111_15 * my * mx;
+    R t[6] = {R(0.), R(0.), R(0.), R(0.), R(0.), R(0.)};
+    if (P.fm) {
+        t[0] = mt.l100_15 * (mx * mx - third);
+        t[1] = mt.l100_15 * (my * my - third);
+        t[2] = mt.l100_15 * (mz * mz - third);
+        t[3] = mt.l111_15 * my * mz;
+        t[4] = mt.l111_15 * mx * mz;
+        t[5] = mt.l111_15 * my * mx;
+    }
     // electrostriction, added in the same order.  Evaluated also without
     // ferroelectrics (p = 0): the terms are then zeros, but adding +0 turns a
     // -0 magnetostriction term (e.g. l111 my mz with mz = 0, my < 0) into +0,
@@ -726,10 +727,8 @@ __device__ __forceinline__ void elastic_tile_body(const Params& P, const StageIO
                     }
 #pragma unroll
                     for (int a = 0; a < 3; a++) tz[a] = qdivR((s2[a] - s1[a]), P.dz, P.rdz, P.f.rdz);
-                    // cell strain for the magnetic kernels and, in the FP64 form,
-                    // the TDGL kernel (the mixed form's TDGL kernel forms its own
-                    // from u: fewer bytes, and its FP32 registers hold the stencil)
-                    if (want_strain && (sm.mat()[id - 1].flags & (MF_FM | MF_AFM | (is_mixed<R>::value ? 0u : MF_FE)))) {
+                    // cell strain for the magnetic kernels (the TDGL kernel forms its own)
+                    if (want_strain && (sm.mat()[id - 1].flags & (MF_FM | MF_AFM))) {
                         R e[6];
                         e[0] = (me.gm(0, 0) + me.gp(0, 0)) / R(2.);
                         e[1] = (me.gm(1, 1) + me.gp(1, 1)) / R(2.);

@@ -122,6 +122,10 @@ struct gf_engine {
     int el_nmat = 0;                   // materials staged by k_elastic_tile
     size_t el_smem = 0;                // its dynamic shared memory
     bool el_cubic = false;             // every material has the cubic stiffness pattern
+    // every cell is material 1, whose constants the kernels of such runs take by value
+    bool uni = false;
+    DevMat um = {};
+    DevMatT<float> um_f = {};
     double* liao_hist = nullptr; double* liao_last = nullptr;
     double* scratch = nullptr;             // output staging (scratch_main doubles), then reduction partials
     size_t scratch_main = 0;
@@ -845,6 +849,11 @@ int set_elastic_smem(gf_engine* eng, int smem) {
     return GF_OK;
 }
 
+template <class R>
+const DevMatT<R>& uni_mat(const gf_engine* eng) {
+    if constexpr (is_mixed<R>::value) return eng->um_f; else return eng->um;
+}
+
 #ifndef GF_MIXED_TU
 int setup_elastic_tile(gf_engine* eng) {
     const Params& P = eng->P;
@@ -999,8 +1008,10 @@ template <int S, class R>
 int enqueue_fe(gf_engine* eng, const StageIOT<R>& io, cudaStream_t st) {
     const Params& P = eng->P;
     const dim3 g(blocks_for((long)P.ny * P.nz, kThreads), (unsigned)P.nx);
-    if (P.flexo) GF_CU(klaunch(eng, "k_fe", k_fe<S, R, true>, g, dim3(kThreads), 0, st, P, io));
-    else GF_CU(klaunch(eng, "k_fe", k_fe<S, R, false>, g, dim3(kThreads), 0, st, P, io));
+    const DevMatT<R>& um = uni_mat<R>(eng);
+    if (P.flexo) GF_CU(klaunch(eng, "k_fe", k_fe<S, R, true, false>, g, dim3(kThreads), 0, st, P, io, um));
+    else if (eng->uni && (um.flags & MF_FE)) GF_CU(klaunch(eng, "k_fe", k_fe<S, R, false, true>, g, dim3(kThreads), 0, st, P, io, um));
+    else GF_CU(klaunch(eng, "k_fe", k_fe<S, R, false, false>, g, dim3(kThreads), 0, st, P, io, um));
     return GF_OK;
 }
 
@@ -1030,8 +1041,8 @@ int enqueue_stage(gf_engine* eng, int parity) {
     cudaStream_t st = eng->stream;
     const unsigned bn = blocks_for(P.n, kThreads);
     // The physics of a stage read only the stage inputs, except for these
-    // dependencies: the LLG and (FP64) TDGL kernels read the cell strain the
-    // elastic tile writes, flexoelectric runs read k_flexo_prep's arrays, the
+    // dependencies: the LLG kernels read the cell strain the elastic kernel
+    // writes, flexoelectric runs read k_flexo_prep's arrays, the
     // Maxwell update reads the LLG increment (M-sourced current, spin
     // pumping), and the PEC kernel clears the step-start E that the TDGL
     // kernel reads at stage 1.  So the elastic chain runs on the engine
@@ -1051,7 +1062,6 @@ int enqueue_stage(gf_engine* eng, int parity) {
     const bool mag = P.fm || P.afm;
     const bool em_after_llg = P.em && mag && (P.em_fromM || P.spin);
     const bool em_after_fe = P.em && P.fe && P.pec;
-    const bool fe_after_tile = P.fe && P.elastic && P.elasto_on && !is_mixed<R>::value;
     GF_CU(rec(ev_start, st));
     if (P.em && !em_after_llg && !em_after_fe) {
         GF_CU(wait_(s_em, ev_start, 0));
@@ -1062,7 +1072,7 @@ int enqueue_stage(gf_engine* eng, int parity) {
         GF_CU(klaunch(eng, "k_flexo_prep", k_flexo_prep<R>, dim3(blocks_for((long)P.ny * P.nz, kThreads), (unsigned)P.nx),
                       dim3(kThreads), 0, st, P, io));
     GF_CU(rec(ev_pre, st));
-    if (P.fe && !fe_after_tile) {
+    if (P.fe) {
         GF_CU(wait_(s_fe, ev_pre, 0));
         GF_TRY((enqueue_fe<S, R>(eng, io, s_fe)));
         GF_CU(rec(ev_fe, s_fe));
@@ -1079,11 +1089,6 @@ int enqueue_stage(gf_engine* eng, int parity) {
                                 eng->el_chunk, eng->el_nmat, tm));
     }
     GF_CU(rec(ev_tile, st));
-    if (P.fe && fe_after_tile) {
-        GF_CU(wait_(s_fe, ev_tile, 0));
-        GF_TRY((enqueue_fe<S, R>(eng, io, s_fe)));
-        GF_CU(rec(ev_fe, s_fe));
-    }
     if (mag) {
         GF_CU(wait_(s_llg, ev_tile, 0));
         if (P.fm) GF_CU(klaunch<true>(eng, "k_llg_fm", k_llg_fm<S, R>, dim3(blocks_for(P.fm_bj * P.fm_bk, kThreads), (unsigned)P.fm_bi),
@@ -1852,9 +1857,8 @@ int create_from(gf_engine* eng, const std::string& dir, int device, int precisio
         // Without magnets the elastic chain of the engine stream (tile, RK
         // update) is the longest of a stage and goes first, then the
         // Maxwell update and the TDGL kernel in the order measured faster
-        // for each form (128^3 ferroelectric, ms per step: FP64 2.453 ->
-        // 2.357 with Maxwell before TDGL, which waits for the tile there;
-        // FP32 1.422 -> 1.354 with TDGL before Maxwell).  With magnets the
+        // for each form (128^3 ferroelectric, ms per step: FP64 1.513 with
+        // Maxwell before TDGL, 1.530 the other way; FP32 TDGL before Maxwell).  With magnets the
         // LLG and Maxwell kernels wait for the tile and RK update is off the
         // critical path: equal priorities (128x128x96 magnetoelastic: the
         // elastic-first order measured 0.878 -> 0.905 ms FP32, 1.491 ->
@@ -1880,6 +1884,11 @@ int create_from(gf_engine* eng, const std::string& dir, int device, int precisio
     }
 
     // materials
+    if (!d.mats.empty()) {
+        eng->uni = std::all_of(d.material_cell.begin(), d.material_cell.end(), [](auto id) { return id == 1; });
+        eng->um = make_devmat(d.mats[0], d.dt);
+        eng->um_f = devmat_f32(eng->um);
+    }
     GF_TRY(dalloc_n(eng, &eng->mid, (size_t)n));
     GF_CU(cudaMemcpyAsync(eng->mid, d.material_cell.data(), (size_t)n, cudaMemcpyHostToDevice, eng->stream));
     std::vector<DevMat> dm(d.mats.size());
@@ -2003,8 +2012,7 @@ int create_from(gf_engine* eng, const std::string& dir, int device, int precisio
     if (d.elastodynamics)
         for (int a = 0; a < 9; a++) GF_TRY(dalloc_r(eng, &eng->fg[a], (size_t)n));
     // the crystal-frame cell strain the elastic tile hands to the LLG kernels
-    // and to the FP64 TDGL kernel
-    if (d.elastodynamics && P.elasto_on && (P.fm || P.afm || (P.fe && !eng->mixed)))
+    if (d.elastodynamics && P.elasto_on && (P.fm || P.afm))
         for (int a = 0; a < 6; a++) GF_TRY(dalloc_r(eng, &eng->strain_c[a], (size_t)n));
     // flexoelectricity: global-frame cell strain and eigenstrain p-gradients
     // of the stage state (k_flexo_prep)
@@ -3536,6 +3544,8 @@ int batch_upload(gf_batch* b, const std::vector<int>& ch) {
         t.nmat = (int)e->deck.mats.size();
         t.el_chunk = ch[i];
         t.el_cubic = e->el_cubic ? 1 : 0;
+        t.uni = e->uni && (e->um_f.flags & MF_FE) ? 1 : 0;
+        t.um = e->um_f;
         t.step = e->step_ctr;
     }
     std::vector<BatchItem> A, At, Ae, Af, B, C, D;

@@ -190,8 +190,11 @@ __device__ __forceinline__ void fe_dq(const Params& P, const StageIOT<R>& io, in
             exx = edyn[0]; eyy = edyn[1]; ezz = edyn[2]; eyz = edyn[3]; exz = edyn[4]; exy = edyn[5];
         }
         if (P.elasto_back) {
-            R e0[6];
-            eigen_crt(P, io, c, e0);
+            R e0[6], es[6] = {R(0.), R(0.), R(0.), R(0.), R(0.), R(0.)};
+            R mx = R(0.), my = R(0.), mz = R(0.);
+            if (P.fm) glb2crt(P, io.m_in.c[0][c], io.m_in.c[1][c], io.m_in.c[2][c], mx, my, mz);
+            if (io.eig0_c[0]) for (int a = 0; a < 6; a++) es[a] = io.eig0_c[a][c];
+            eigen_terms(P, io, c, mt, mx, my, mz, px, py, pz, es, e0);
             exx0 = e0[0]; eyy0 = e0[1]; ezz0 = e0[2]; eyz0 = e0[3]; exz0 = e0[4]; exy0 = e0[5];
         }
         if (P.elastostatic) {
@@ -425,7 +428,9 @@ __device__ __forceinline__ void fe_rk(const Params& P, const StageIOT<R>& io, in
     }
 }
 
-template <int S, class R, bool FX>
+template <int S, class R, bool FX, bool UNI>
+// UNI: every cell is material 1, whose constants are um (constant bank
+// operands in place of ~30 loads per cell, and no material ids).
 // FX: the run has flexoelectricity (the polarisation- and strain-gradient
 // terms of get_dq_RK*, ferroelectric_solver.cpp:800-833).
 // FP64 (256, 3): 80 registers, 24 resident warps per SM (measured best of 2-4
@@ -434,20 +439,21 @@ template <int S, class R, bool FX>
 // (FP64) per step on the 128^3 ferroelectric workload, against 0.79 at
 // (256, 2); FP32 0.363 ms per step at (256, 5), against 0.381 at 4 (64
 // registers), 0.368 at 6 (spills) and 0.49 at 3
-__device__ __forceinline__ void fe_body(const Params& P, const StageIOT<R>& io, int bx, int by) {
+__device__ __forceinline__ void fe_body(const Params& P, const StageIOT<R>& io, const DevMatT<R>& um, int bx, int by) {
     const int nx = P.nx, ny = P.ny, nz = P.nz;
     const int t = bx * blockDim.x + threadIdx.x;
     if (t >= ny * nz) return;
     const int i = by, j = t / nz, k = t - (t / nz) * nz;
     const int c = (i * ny + j) * nz + k;
-    const uint8_t id = io.mid[c];
+    uint8_t id = 1;
+    if constexpr (!UNI) id = io.mid[c];
     R dq[3] = {R(0.), R(0.), R(0.)};
 
     // material classes from the run's bitmask: no table load on the path to
     // the neighbour loads
-    auto fe_id = [&](uint8_t q) { return q != 0 && ((P.fe_mask >> (q - 1)) & 1u); };
+    auto fe_id = [&](uint8_t q) { return UNI || (q != 0 && ((P.fe_mask >> (q - 1)) & 1u)); };
     if (fe_id(id)) {
-        const DevMatT<R>& mt = io.mats[id - 1];
+        const DevMatT<R>& mt = UNI ? um : io.mats[id - 1];
         const R pxg = io.p_in.c[0][c], pyg = io.p_in.c[1][c], pzg = io.p_in.c[2][c];
 
         // ---- Laplacian with mirror condition at FE interfaces ----
@@ -466,7 +472,10 @@ __device__ __forceinline__ void fe_body(const Params& P, const StageIOT<R>& io, 
             for (int f = 0; f < 6; f++) pn[a][f] = io.p_in.c[a][nb[f]];
         uint8_t idn[6];
 #pragma unroll
-        for (int f = 0; f < 6; f++) idn[f] = io.mid[nb[f]];
+        for (int f = 0; f < 6; f++) {
+            idn[f] = 1;
+            if constexpr (!UNI) idn[f] = io.mid[nb[f]];
+        }
         const bool surf[6] = {(i == 0 && !P.per_x) || !fe_id(idn[0]),
                               (i == nx - 1 && !P.per_x) || !fe_id(idn[1]),
                               (j == 0 && !P.per_y) || !fe_id(idn[2]),
@@ -498,18 +507,12 @@ __device__ __forceinline__ void fe_body(const Params& P, const StageIOT<R>& io, 
 
         R edyn[6] = {R(0), R(0), R(0), R(0), R(0), R(0)};
         if (P.elasto_on && P.elastic) {
-            if constexpr (is_mixed<R>::value) {
-                // mixed form: from the stage displacement (the values
-                // k_elastic_tile forms), 12 bytes of u instead of 24 of strain
-                const bool solid_nb[6] = {idn[0] != 0, idn[1] != 0, idn[2] != 0, idn[3] != 0, idn[4] != 0, idn[5] != 0};
-                fe_cell_strain(P, io, i, j, k, c, nb, solid_nb, true, edyn);
-            } else {
-                // FP64: written by k_elastic_tile earlier in the same stage
-                // (forming it here costs the FP64 kernel more in registers
-                // and latency than the 48 bytes it saves)
-#pragma unroll
-                for (int q = 0; q < 6; q++) edyn[q] = io.strain_c[q][c];
-            }
+            // from the stage displacement (the values the elastic kernel forms):
+            // 24 bytes of u per cell instead of 48 of strain written there and
+            // read here (FP64, 128^3 ferroelectric step 1.566 -> 1.528 ms), and
+            // no wait for that kernel
+            const bool solid_nb[6] = {idn[0] != 0, idn[1] != 0, idn[2] != 0, idn[3] != 0, idn[4] != 0, idn[5] != 0};
+            fe_cell_strain(P, io, i, j, k, c, nb, solid_nb, true, edyn);
         }
         fe_dq<S, R, FX>(P, io, i, j, k, c, mt, pxg, pyg, pzg, lap, edyn, d2s, dp, nb, idn, dq);
     }
@@ -518,9 +521,10 @@ __device__ __forceinline__ void fe_body(const Params& P, const StageIOT<R>& io, 
 
 
 // block (bx, by): 256 cells of the (j, k) plane bx of x-plane by
-template <int S, class R = double, bool FX = false>
-__global__ void __launch_bounds__(256, is_mixed<R>::value ? GF_FE_MINB_F32 : GF_FE_MINB_F64) k_fe(Params P, StageIOT<R> io) {
-    fe_body<S, R, FX>(P, io, blockIdx.x, blockIdx.y);
+template <int S, class R, bool FX, bool UNI>
+__global__ void __launch_bounds__(256, is_mixed<R>::value ? GF_FE_MINB_F32 : GF_FE_MINB_F64)
+    k_fe(const __grid_constant__ Params P, const __grid_constant__ StageIOT<R> io, const __grid_constant__ DevMatT<R> um) {
+    fe_body<S, R, FX, UNI>(P, io, um, blockIdx.x, blockIdx.y);
 }
 
 }  // namespace gf

@@ -52,8 +52,8 @@ struct StageIOT {
     // cell's -d face
     R* fg[9];
     // crystal-frame cell strain of the stage displacement (Dexx_crt ...),
-    // written by k_elastic_tile for ferromagnetic and ferroelectric cells and
-    // read by the LLG and TDGL kernels of the same stage; null when unused
+    // written by the elastic kernel for magnetic cells and read by the LLG
+    // kernels of the same stage; null when unused
     R* strain_c[6];
     // optional static inputs (null when absent): static strain and static
     // eigenstrain in the crystal frame

@@ -1,0 +1,111 @@
+"""GPU tests of the specialised stage kernels against the general ones they
+stand in for, over the forms they accept.
+
+A deck and the same deck on the general path give the same physics: two
+materials with the same constants keep the TDGL and column kernels from the
+single-material form, an identity frame rotation (if_OrientRotate with Tg2c = 1) keeps the elastic
+stage on k_elastic_tile, and a Drude pole in a material that no cell has keeps
+the Yee update on k_em_fused.  The convolution is compared with the numpy
+restatement (oracle/restate_fm.py).
+
+Tolerances: the paths order the same sums differently, so fields differ by a
+few rounding errors of their terms.  After three steps an FP64 field carries
+of order 1e-15 x the cancellation in a stress or curl difference (up to ~1e2
+for the random fields here): 1e-12.  FP32: 1e-7 x the same: 2e-5.
+"""
+import dataclasses
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+TOL = {"fp64": 1e-12, "mixed": 2e-5}
+FIELDS = ("m", "m_afm1", "p", "q", "u", "v", "force_store", "Ex", "Ey", "Ez", "Hx", "Hy", "Hz")
+
+
+def _run(gf, d, precision, steps=3):
+    out = {}
+    with gf.Engine.from_params(d, device=0, precision=precision) as e:
+        e.advance(steps)
+        for f in FIELDS:
+            try:
+                out[f] = e.download(f)
+            except gf.GFError:
+                pass
+        e.check_finite()
+    return out
+
+
+def _same(a, b, tol):
+    assert a.keys() == b.keys()
+    for f in a:
+        n = np.linalg.norm(b[f])
+        d = np.linalg.norm(a[f] - b[f])
+        assert np.isfinite(d) and d <= tol * n, (f, d / n if n else d)
+
+
+def _unit(rng, shape):
+    v = rng.standard_normal((3,) + shape)
+    return v / np.linalg.norm(v, axis=0)
+
+
+def _moving(d, seed):
+    """Random displacement, velocity and order parameters of the deck's cells."""
+    rng = np.random.default_rng(seed)
+    sh = (d.nx, d.ny, d.nz)
+    mc = d.material_cell()
+    solid = mc != 0
+    if d.elastic:
+        d.u0 = 1e-13 * rng.standard_normal((3,) + sh) * solid
+        d.v0 = 1e-2 * rng.standard_normal((3,) + sh) * solid
+
+    def has(flag):
+        return np.isin(mc, [q + 1 for q, m in enumerate(d.materials) if getattr(m, flag)])
+    d.m0 = d.p0 = d.q0 = None
+    if has("fm").any():
+        d.m0 = _unit(rng, sh) * has("fm")
+    if has("afm").any():
+        d.afm0 = np.concatenate([_unit(rng, sh) * has("afm"), _unit(rng, sh) * has("afm")])
+    if has("fe").any():
+        d.p0 = 0.05 * rng.standard_normal((3,) + sh) * has("fe")
+        d.q0 = np.zeros_like(d.p0)
+    return d
+
+
+def _fe(gf, nx, ny, nz, **kw):
+    d = gf.decks.preset_ferroelectric(nx=nx, ny=ny, nz=nz, steps=10)
+    for k, v in kw.items():
+        setattr(d, k, v)
+    return d
+
+
+def _me(gf, nx, ny, nz, sub, film, **kw):
+    d = gf.decks.preset_magnetoelastic(nx=nx, ny=ny, nz=nz, sub=sub, film=film, steps=10)
+    for k, v in kw.items():
+        setattr(d, k, v)
+    return d
+
+
+def _scattered(gf, nx, ny, nz, mats, seed, **kw):
+    d = _fe(gf, nx, ny, nz)
+    d.materials = mats
+    rng = np.random.default_rng(seed)
+    d.struct = rng.integers(0, len(mats) + 1, (nx, ny, nz)).astype(np.uint8)
+    d.layers = [(nz, 1)]
+    for k, v in kw.items():
+        setattr(d, k, v)
+    return d
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("shape", [(1, 5, 5), (9, 21, 13), (12, 33, 32)])
+@pytest.mark.parametrize("elastic", [True, False])
+def test_tdgl_of_one_material_equals_two_alike(gf, shape, elastic, precision):
+    d = _fe(gf, *shape)
+    if not elastic:
+        d = dataclasses.replace(d, elastic=False, elasto_back=False, elasto_on=False)
+    d = _moving(d, 31)
+    g = dataclasses.replace(d, materials=[d.materials[0]] * 2)
+    g.struct = np.random.default_rng(37).integers(1, 3, shape).astype(np.uint8)
+    _same(_run(gf, d, precision), _run(gf, g, precision), TOL[precision])
