@@ -19,13 +19,13 @@
 // on the host, longest kinds first; each block reads its engine's parameters
 // and stage buffers from the engine table (read-only, cached) and runs the
 // kind's body —
-// the same device functions the per-engine kernels run (elastic_tile_body,
-// fe_body, em_fused_body, elastic_rk_body, em_mur_body, elastic_bc_body), so
+// the same device functions the per-engine kernels run ( elastic_col_body or
+// elastic_tile_body, fe_body, em_fused_body, elastic_rk_body, em_mur_body, elastic_bc_body), so
 // the arithmetic is the per-engine kernels'.  Small grids share the GPU
 // within one launch instead of occupying it one after another.
 #pragma once
 
-#include "gf_elastic.cuh"
+#include "gf_column.cuh"
 #include "gf_em.cuh"
 #include "gf_fe.cuh"
 
@@ -41,6 +41,8 @@ struct BatchInst {
     int ncls, nmat, el_chunk, el_cubic;
     int uni;                           // every cell is ferroelectric material 1, um
     DevMatT<float> um;
+    int el_col, el_pm;                 // k_elastic_col's form of the stress divergence, on tiles of geom
+    ColGeom geom;
     unsigned long long* step;          // the engine's step counter
 };
 
@@ -48,6 +50,21 @@ struct BatchInst {
 struct BatchItem {
     int inst, kind, bx, by, bz;
 };
+
+// the stress divergence of a tile item, in the form the engine alone uses
+template <int S>
+__device__ __forceinline__ void batch_tile(const BatchInst& g, const StageIOT<float>& io, const BatchItem it, const ETileMaps& tm,
+                                           unsigned char* smem_raw) {
+    if (g.el_col) {
+        const ColMat<float> none{};
+        if (g.el_pm == CE_P) elastic_col_body<float, false, CE_P, kColBatchThreads>(g.P, io, g.geom, g.nmat, none, it.bx, it.by, it.bz, smem_raw);
+        else elastic_col_body<float, false, CE_ANY, kColBatchThreads>(g.P, io, g.geom, g.nmat, none, it.bx, it.by, it.bz, smem_raw);
+    } else if (g.el_cubic) {
+        elastic_tile_body<S, true, float>(g.P, io, g.el_chunk, g.nmat, tm, it.bx, it.by, it.bz, smem_raw);
+    } else {
+        elastic_tile_body<S, false, float>(g.P, io, g.el_chunk, g.nmat, tm, it.bx, it.by, it.bz, smem_raw);
+    }
+}
 
 // the TDGL update of an item, in the form the engine alone uses
 template <int S>
@@ -71,8 +88,7 @@ __device__ __forceinline__ void batch_item(const BatchInst* __restrict__ insts, 
     const Params& P = g.P;
     const StageIOT<float>& io = g.io[parity][S];
     auto tile = [&]() {
-        if (g.el_cubic) elastic_tile_body<S, true, float>(P, io, g.el_chunk, g.nmat, tm, it.bx, it.by, it.bz, smem_raw);
-        else elastic_tile_body<S, false, float>(P, io, g.el_chunk, g.nmat, tm, it.bx, it.by, it.bz, smem_raw);
+        batch_tile<S>(g, io, it, tm, smem_raw);
     };
     auto yee = [&]() {
         EmMat<float>* mt = reinterpret_cast<EmMat<float>*>(smem_raw);
@@ -154,8 +170,7 @@ __device__ __noinline__ void batch_kind_call(const BatchInst* __restrict__ insts
     const Params& P = g.P;
     const StageIOT<float>& io = g.io[parity][S];
     if constexpr (K == BK_TILE) {
-        if (g.el_cubic) elastic_tile_body<S, true, float>(P, io, g.el_chunk, g.nmat, *tm, it.bx, it.by, it.bz, smem_raw);
-        else elastic_tile_body<S, false, float>(P, io, g.el_chunk, g.nmat, *tm, it.bx, it.by, it.bz, smem_raw);
+        batch_tile<S>(g, io, it, *tm, smem_raw);
     } else if constexpr (K == BK_EM) {
         EmMat<float>* mt = reinterpret_cast<EmMat<float>*>(smem_raw);
         EmCls<float>* cl = reinterpret_cast<EmCls<float>*>(smem_raw + kMaxMat * sizeof(EmMat<float>));

@@ -33,6 +33,7 @@
 #include "gf_launch.cuh"
 #include "gf_state.cuh"
 #include "gf_elastic.cuh"
+#include "gf_column.cuh"
 #include "gf_llg.cuh"
 #include "gf_fe.cuh"
 #include "gf_em.cuh"
@@ -126,6 +127,9 @@ struct gf_engine {
     bool uni = false;
     DevMat um = {};
     DevMatT<float> um_f = {};
+    // k_elastic_col runs the stress divergence (col_path), and its tile
+    bool el_col = false;
+    ColGeom el_geom = {};
     double* liao_hist = nullptr; double* liao_last = nullptr;
     double* scratch = nullptr;             // output staging (scratch_main doubles), then reduction partials
     size_t scratch_main = 0;
@@ -201,6 +205,7 @@ struct gf_engine {
 int gf_mixed_enqueue_step(gf_engine* eng, int parity);                 // kernels of one step, mixed form
 int gf_mixed_enqueue_stage(gf_engine* eng, int parity, int s);         // kernels of stage s (0..3), mixed form
 int gf_mixed_elastic_setup(gf_engine* eng, int smem, int* per_sm);   // shared-memory opt-in, occupancy
+int gf_mixed_col_setup(gf_engine* eng);                                 // the same for k_elastic_col, and its tile
 int gf_mixed_time_tile(gf_engine* eng, int reps, float* ms);          // stage-1 elastic tile, mean ms per launch
 int gf_mixed_adj_elastic(gf_engine* eng, int s, int rk, const StageIOT<float>& io);  // adjoint: FP32 elastic tile / RK of stage s
 int gf_mixed_batch_attr(size_t smem);                                   // shared-memory opt-in of the batch phase kernels
@@ -849,12 +854,85 @@ int set_elastic_smem(gf_engine* eng, int smem) {
     return GF_OK;
 }
 
+// the fields the eigenstrain of engine e reads now (a static eigenstrain may
+// arrive after creation)
+inline int col_pm(const gf_engine* e) {
+    const Params& P = e->P;
+    if (!P.elasto_back || P.afm || P.flexo || e->es_eig[0]) return CE_ANY;
+    return (P.fe && !P.fm) ? CE_P : ((P.fm && !P.fe) ? CE_M : CE_ANY);
+}
+// calls fn with the instantiation of k_elastic_col for uni and pm
+template <class R, class F>
+auto col_dispatch(bool uni, int pm, F fn) {
+    if (uni) {
+        if (pm == CE_P) return fn(k_elastic_col<R, true, CE_P>);
+        if (pm == CE_M) return fn(k_elastic_col<R, true, CE_M>);
+        return fn(k_elastic_col<R, true, CE_ANY>);
+    }
+    if (pm == CE_P) return fn(k_elastic_col<R, false, CE_P>);
+    if (pm == CE_M) return fn(k_elastic_col<R, false, CE_M>);
+    return fn(k_elastic_col<R, false, CE_ANY>);
+}
 template <class R>
 const DevMatT<R>& uni_mat(const gf_engine* eng) {
     if constexpr (is_mixed<R>::value) return eng->um_f; else return eng->um;
 }
+template <class R>
+ColMat<R> col_um(const gf_engine* eng) { return col_mat(uni_mat<R>(eng)); }
+inline dim3 col_grid(const gf_engine* eng) {
+    const ColGeom& g = eng->el_geom;
+    return dim3((unsigned)g.tk, (unsigned)g.tj, (unsigned)((eng->P.nx + g.chunk - 1) / g.chunk));
+}
+
+// shared-memory opt-in of k_elastic_col, its tile and x-chunk for the grid
+template <class R>
+int col_setup(gf_engine* eng) {
+    const int nmat = eng->el_nmat;
+    int sms = 1;
+    GF_CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, eng->device));
+    // a function's attribute is the process's: set it for the most materials a
+    // deck can have, so that engines with fewer do not lower it
+    for (int pm : {CE_P, CE_M, CE_ANY})
+        GF_CU(col_dispatch<R>(eng->uni, pm, [&](auto k) {
+            return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)col_smem_bytes<R>(kColMaxThreads<R>, kMaxMat));
+        }));
+    std::vector<long> memo(kColMaxThreads<R> + 1, -1);
+    auto slots = [&](int threads) -> long {
+        if (memo[threads] < 0) {
+            int per = 0;
+            const cudaError_t e = col_dispatch<R>(eng->uni, col_pm(eng), [&](auto k) {
+                return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, threads, col_smem_bytes<R>(kColMaxThreads<R>, nmat));
+            });
+            memo[threads] = e == cudaSuccess ? (long)per * sms : 0;
+        }
+        return memo[threads];
+    };
+    eng->el_geom = col_geom<R>(eng->P, kColMaxThreads<R>, sms, slots);
+    if (eng->el_geom.threads < 1) { eng->err = "elastic column tile does not fit on an SM"; return GF_ECUDA; }
+    eng->el_chunk = eng->el_geom.chunk;
+    return GF_OK;
+}
+
+// one launch of k_elastic_col on the stage buffers io
+template <class R>
+cudaError_t col_launch(gf_engine* eng, const StageIOT<R>& io, cudaStream_t st, bool counted) {
+    const ColGeom& g = eng->el_geom;
+    const size_t sm = col_smem_bytes<R>(kColMaxThreads<R>, eng->el_nmat);
+    return col_dispatch<R>(eng->uni, col_pm(eng), [&](auto k) {
+        return counted ? klaunch<true>(eng, "k_elastic", k, col_grid(eng), dim3(g.threads), sm, st, eng->P, io, g, eng->el_nmat, col_um<R>(eng))
+                       : launch_tiled(k, col_grid(eng), dim3(g.threads), sm, st, eng->P, io, g, eng->el_nmat, col_um<R>(eng));
+    });
+}
 
 #ifndef GF_MIXED_TU
+// Decks k_elastic_col covers: every material cubic in the unrotated frame, no
+// surface traction source, and no column where the reference's +z neighbour
+// of k = ny-1 is k = 0 (ny < nz).  The others keep k_elastic_tile.
+bool col_path(const gf_engine* eng) {
+    const Params& P = eng->P;
+    return eng->el_cubic && !P.rot && !(P.strain_pulse && P.strain_type == 3) && P.ny >= P.nz;
+}
+
 int setup_elastic_tile(gf_engine* eng) {
     const Params& P = eng->P;
     eng->el_nmat = (int)eng->deck.mats.size();
@@ -865,6 +943,10 @@ int setup_elastic_tile(gf_engine* eng) {
         for (int a = 0; a < 6; a++)
             for (int b = 0; b < 6; b++)
                 if (!((a < 3 && b < 3) || a == b) && m.cij[a][b] != 0.) eng->el_cubic = false;
+    eng->el_col = col_path(eng);
+    if (eng->el_col) {
+        return eng->mixed ? gf_mixed_col_setup(eng) : col_setup<double>(eng);
+    }
     int per_sm = 1, sms = 1;
     if (eng->mixed) {
         GF_TRY(gf_mixed_elastic_setup(eng, smem, &per_sm));
@@ -1077,7 +1159,9 @@ int enqueue_stage(gf_engine* eng, int parity) {
         GF_TRY((enqueue_fe<S, R>(eng, io, s_fe)));
         GF_CU(rec(ev_fe, s_fe));
     }
-    if (P.elastic) {
+    if (P.elastic && eng->el_col) {
+        GF_CU(col_launch<R>(eng, io, st, true));
+    } else if (P.elastic) {
         const dim3 grid((P.nz + etile::TK - 1) / etile::TK, (P.ny + etile::TJ - 1) / etile::TJ,
                         (P.nx + eng->el_chunk - 1) / eng->el_chunk);
         const ETileMaps& tm = eng->etm[parity][S];
@@ -1149,6 +1233,7 @@ int time_tile_t(gf_engine* eng, int reps, float* ms) {
     GF_CU(cudaEventCreate(&b));
     const ETileMaps& tm = eng->etm[(int)(eng->steps_done & 1ull)][0];
     auto one = [&]() {
+        if (eng->el_col) return col_launch<R>(eng, io, eng->stream, false);
         return eng->el_cubic ? launch_tiled(k_elastic_tile<0, true, R>, grid, dim3(etile::NT), eng->el_smem, eng->stream, P, io,
                                             eng->el_chunk, eng->el_nmat, tm)
                              : launch_tiled(k_elastic_tile<0, false, R>, grid, dim3(etile::NT), eng->el_smem, eng->stream, P, io,
@@ -1197,6 +1282,8 @@ int gf_mixed_elastic_setup(gf_engine* eng, int smem, int* per_sm) {
     return GF_OK;
 }
 
+int gf_mixed_col_setup(gf_engine* eng) { return col_setup<float>(eng); }
+
 int gf_mixed_time_tile(gf_engine* eng, int reps, float* ms) { return time_tile_t<float>(eng, reps, ms); }
 
 // the FP32 elastic tile (rk = 0) or RK update (rk = 1) of stage s on the
@@ -1212,6 +1299,10 @@ int adj_elastic_f32(gf_engine* eng, int rk, const StageIOT<float>& io) {
         Params Pa = P;
         Pa.el_bc_fused = 0;
         GF_CU(launch(k_elastic_rk<S, float>, dim3(blocks_for(P.n, 2 * kThreads)), dim3(kThreads), 0, eng->stream, Pa, io));
+        return GF_OK;
+    }
+    if (eng->el_col) {
+        GF_CU(col_launch<float>(eng, io, eng->stream, false));
         return GF_OK;
     }
     ETileMaps tm;
@@ -1788,7 +1879,7 @@ int etile_maps(gf_engine* eng) {
     if (!eng->tma_err) GF_TRY(dalloc_n(eng, &eng->tma_err, 1));
     for (auto& row : eng->etm)
         for (ETileMaps& m : row) { std::memset(&m, 0, sizeof(m)); m.err = eng->tma_err; m.on = 0; }
-    if (!P.elastic) return GF_OK;
+    if (!P.elastic || eng->el_col) return GF_OK;
     // GOFERRO_TILE_TMA=0 keeps every block on the cp.async staging (the
     // tests check that both stagings give the same bits)
     if (const char* v = std::getenv("GOFERRO_TILE_TMA"))
@@ -3454,13 +3545,13 @@ int autotune_tile(gf_batch* b, gf_engine* e) {
     int best = base;
     float best_ms = -1.f;
     for (int L : cand) {
-        e->el_chunk = L;
+        e->el_chunk = e->el_geom.chunk = L;
         float ms = 0.f;
         int rc = e->mixed ? gf_mixed_time_tile(e, 5, &ms) : time_tile_t<double>(e, 5, &ms);
-        if (rc != GF_OK) { e->el_chunk = base; return batch_fail(b, e, rc); }
+        if (rc != GF_OK) { e->el_chunk = e->el_geom.chunk = base; return batch_fail(b, e, rc); }
         if (best_ms < 0.f || ms < best_ms) { best_ms = ms; best = L; }
     }
-    e->el_chunk = best;
+    e->el_chunk = e->el_geom.chunk = best;
     e->graphs_ready = false;          // the engine's own graphs hold the old grid
     for (int p = 0; p < 2; p++) {
         if (e->gexec[p]) { cudaGraphExecDestroy(e->gexec[p]); e->gexec[p] = nullptr; }
@@ -3485,6 +3576,13 @@ std::string batch_phase_blocker(const gf_engine* e) {
     return "";
 }
 
+// column tile of engine e's work items: at most a batch block's threads
+ColGeom batch_geom(const gf_engine* e, int chunk) {
+    if (!e->el_col) return ColGeom{};
+    // the items of all engines share an SM's slots
+    return col_geom<float>(e->P, kColBatchThreads, 148, [](int) { return 148L * 3; }, std::min(chunk, (int)e->P.nx));
+}
+
 // the work items of every engine at elastic x-chunk ch[i]: phase A's tile,
 // Yee and TDGL items (A = all three, tiles first: the longest items); B the
 // RK update, C the elastic boundary planes; an engine's Mur directions in
@@ -3498,7 +3596,10 @@ void batch_items(const gf_batch* b, const std::vector<int>& ch, std::vector<Batc
         const int in = (int)i;
         const long nx = P.nx, ny = P.ny, nz = P.nz;
         if (P.elastic) {
-            const int gx = (P.nz + etile::TK - 1) / etile::TK, gy = (P.ny + etile::TJ - 1) / etile::TJ;
+            const gf_engine* e = b->engs[i];
+            const ColGeom g = batch_geom(e, ch[i]);
+            const int gx = e->el_col ? g.tk : (P.nz + etile::TK - 1) / etile::TK;
+            const int gy = e->el_col ? g.tj : (P.ny + etile::TJ - 1) / etile::TJ;
             const int gz = (P.nx + ch[i] - 1) / ch[i];
             for (int z = 0; z < gz; z++)
                 for (int y = 0; y < gy; y++)
@@ -3544,8 +3645,11 @@ int batch_upload(gf_batch* b, const std::vector<int>& ch) {
         t.nmat = (int)e->deck.mats.size();
         t.el_chunk = ch[i];
         t.el_cubic = e->el_cubic ? 1 : 0;
+        t.el_col = e->el_col ? 1 : 0;
         t.uni = e->uni && (e->um_f.flags & MF_FE) ? 1 : 0;
         t.um = e->um_f;
+        t.el_pm = col_pm(e);
+        t.geom = batch_geom(e, ch[i]);
         t.step = e->step_ctr;
     }
     std::vector<BatchItem> A, At, Ae, Af, B, C, D;
@@ -4285,6 +4389,10 @@ int adj_el_kernel(gf_adjoint* a, int rk, const StageIOT<double>& io) {
         Params Pa = P;
         Pa.el_bc_fused = 0;
         GF_CU(launch(k_elastic_rk<S, double>, dim3(blocks_for(P.n, kThreads)), dim3(kThreads), 0, eng->stream, Pa, io));
+        return GF_OK;
+    }
+    if (eng->el_col) {
+        GF_CU(col_launch<double>(eng, io, eng->stream, false));
         return GF_OK;
     }
     ETileMaps tm;

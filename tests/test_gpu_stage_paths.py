@@ -98,6 +98,48 @@ def _scattered(gf, nx, ny, nz, mats, seed, **kw):
     return d
 
 
+def _elastic_decks(gf):
+    D = gf.decks
+    damped = dataclasses.replace(D.pto(), mass_damping=1e10, stiff_damping=1e-13, er=7.0)
+    flexo = dataclasses.replace(D.pto(), f11=6.0, f12=3.5, f44=2.5)
+    afm = D.afm_uniaxial(magnetoelastic=True)
+    yig = D.yig(1e-2, magnetoelastic=True)
+    return {
+        # one material, the whole z axis in one tile, tile edges in y, smallest and odd sides
+        "fe_uniform": _fe(gf, 9, 21, 13),
+        "fe_small": _fe(gf, 1, 5, 5),
+        "fe_two_planes": _fe(gf, 2, 7, 6),
+        # several tiles along z and y, with remainders
+        "fe_wide": _fe(gf, 5, 141, 139),
+        # open x and y; periodic z needs ny = nz
+        "fe_open_xy": _fe(gf, 10, 17, 11, periodic=(False, False, False)),
+        "fe_periodic_z": _fe(gf, 6, 12, 12, periodic=(True, True, True), abc_1D=True),
+        # film on a substrate under vacuum, Liao boundary and source
+        "me_film": _me(gf, 7, 20, 20, 9, 7),
+        "me_open_x": _me(gf, 8, 24, 22, 10, 8, periodic=(False, True, False)),
+        # every cell its own material or vacuum, damping, and a work area smaller than the grid
+        "scattered": _scattered(gf, 8, 16, 15, [damped, D.ggg(), D.yig(1e-2, magnetoelastic=True)], 3, magnetostatics=False),
+        "fe_and_fm": _scattered(gf, 6, 12, 9, [D.pto(), D.yig(1e-2, magnetoelastic=True)], 4),
+        "island": _fe(gf, 12, 14, 10, nx_work=7, ny_work=8),
+        "afm": _me(gf, 6, 14, 12, 6, 6, materials=[D.ggg(), afm], magnetostatics=False),
+        "flexo": _fe(gf, 6, 12, 10, materials=[flexo], flexo=True),
+        "no_backaction": _me(gf, 6, 14, 12, 6, 6, elasto_back=False),
+        "no_maxwell": _me(gf, 6, 14, 12, 6, 6, em=False, magnetostatics=False, materials=[D.ggg(), yig]),
+    }
+
+
+ELASTIC = ["fe_uniform", "fe_small", "fe_two_planes", "fe_wide", "fe_open_xy", "fe_periodic_z", "me_film", "me_open_x", "scattered",
+           "fe_and_fm", "island", "afm", "flexo", "no_backaction", "no_maxwell"]
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("name", ELASTIC)
+def test_column_march_equals_the_general_tile(gf, name, precision):
+    d = _moving(_elastic_decks(gf)[name], 17)
+    g = dataclasses.replace(d, Tg2c=np.eye(3))
+    _same(_run(gf, d, precision), _run(gf, g, precision), TOL[precision])
+
+
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
 @pytest.mark.parametrize("shape", [(1, 5, 5), (9, 21, 13), (12, 33, 32)])
 @pytest.mark.parametrize("elastic", [True, False])
