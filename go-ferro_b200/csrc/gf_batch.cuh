@@ -19,8 +19,9 @@
 // on the host, longest kinds first; each block reads its engine's parameters
 // and stage buffers from the engine table (read-only, cached) and runs the
 // kind's body —
-// the same device functions the per-engine kernels run ( elastic_col_body or
-// elastic_tile_body, fe_body, em_fused_body, elastic_rk_body, em_mur_body, elastic_bc_body), so
+// the same device functions the per-engine kernels run (elastic_col_body or
+// elastic_tile_body, fe_body, yee_E_body and yee_H_body or
+// em_fused_body, elastic_rk_body, em_mur_body, elastic_bc_body), so
 // the arithmetic is the per-engine kernels'.  Small grids share the GPU
 // within one launch instead of occupying it one after another.
 #pragma once
@@ -66,6 +67,18 @@ __device__ __forceinline__ void batch_tile(const BatchInst& g, const StageIOT<fl
     }
 }
 
+// the Yee update of an item, in the form the engine alone uses (a batch has
+// no magnetic sources): bz 0 the E edges (or, in one body, both), 1 the H
+// faces; NC as in yee_E_body
+template <int S, bool NC>
+__device__ __forceinline__ void batch_yee(const BatchInst& g, const StageIOT<float>& io, const BatchItem it, EmMat<float>* mt,
+                                          EmCls<float>* cl) {
+    if (!yee_path(g.P)) em_fused_body<S, float>(g.P, io, g.nmat, g.cls, g.ncls, it.bx, it.by, mt, cl);
+    else if (it.bz) yee_H_body<S, float, false, NC>(g.P, io, g.nmat, it.bx, it.by, nullptr);
+    else if (g.P.em_fromP) yee_E_body<S, float, true, false, NC>(g.P, io, g.cls, g.ncls, *g.cls, it.bx, it.by, cl);
+    else yee_E_body<S, float, false, false, NC>(g.P, io, g.cls, g.ncls, *g.cls, it.bx, it.by, cl);
+}
+
 // the TDGL update of an item, in the form the engine alone uses
 template <int S>
 __device__ __forceinline__ void batch_fe(const BatchInst& g, const StageIOT<float>& io, const BatchItem it) {
@@ -93,7 +106,7 @@ __device__ __forceinline__ void batch_item(const BatchInst* __restrict__ insts, 
     auto yee = [&]() {
         EmMat<float>* mt = reinterpret_cast<EmMat<float>*>(smem_raw);
         EmCls<float>* cl = reinterpret_cast<EmCls<float>*>(smem_raw + kMaxMat * sizeof(EmMat<float>));
-        em_fused_body<S, float>(P, io, g.nmat, g.cls, g.ncls, it.bx, it.by, mt, cl);
+        batch_yee<S, true>(g, io, it, mt, cl);
     };
     if constexpr (PH == 0) {
         if (it.kind == BK_TILE) tile();
@@ -174,7 +187,7 @@ __device__ __noinline__ void batch_kind_call(const BatchInst* __restrict__ insts
     } else if constexpr (K == BK_EM) {
         EmMat<float>* mt = reinterpret_cast<EmMat<float>*>(smem_raw);
         EmCls<float>* cl = reinterpret_cast<EmCls<float>*>(smem_raw + kMaxMat * sizeof(EmMat<float>));
-        em_fused_body<S, float>(P, io, g.nmat, g.cls, g.ncls, it.bx, it.by, mt, cl);
+        batch_yee<S, false>(g, io, it, mt, cl);
     } else if constexpr (K == BK_FE) {
         batch_fe<S>(g, io, it);
     } else if constexpr (K == BK_RK) {

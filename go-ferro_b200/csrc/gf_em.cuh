@@ -23,6 +23,7 @@
 // stage; here the box test and the per-stage value are evaluated in-kernel.
 #pragma once
 
+#include "gf_column.cuh"
 #include "gf_state.cuh"
 
 namespace gf {
@@ -44,7 +45,7 @@ struct EmMat {
 // table reads and a division per edge.
 template <class R>
 struct EmCls {
-    R coef, cond, pc;
+    R coef, cond, pc, rpc;     // rpc = 1 / pc
     uint32_t mask;
     int pad_;
 };
@@ -414,6 +415,236 @@ __global__ void __launch_bounds__(256, is_mixed<R>::value ? GF_EM_MINB_F32 : GF_
     __shared__ EmCls<R> cl[kEmMaxCls];
     em_fused_body<S, R>(P, io, nmat, cls_g, ncls, blockIdx.x, blockIdx.y, mt, cl);
 }
+
+// ---------------------------------------------------------------------------
+// The Yee stage update of runs whose E edges have classes and that have no
+// Drude poles, spin pumping or antiferromagnets (the others keep
+// k_em_fused), as one kernel for the E edges and one for the H faces.  The
+// update is bound by the latency of its loads (k_em_fused: 53 % of issue
+// slots, 29 % of DRAM), so what counts is loads in flight: each kernel needs
+// about half the registers and keeps more warps resident, a thread issues
+// all of its loads before it uses one, and the E kernel does not wait for the
+// LLG increment that only the H faces read.  The three edges share the
+// vertex's one wrapped cell (iw, jw, kw) and its lower neighbours, which is
+// what their curls and sources read (9 distinct H values where k_em_fused
+// loads 12 and re-derives the cells per edge), the three faces the vertex's E
+// (9 of 12), and material ids and dM/dt are read only with M sources.
+// Products that feed a sum are fma(), so that the batched kernels give the
+// same bits.
+// ---------------------------------------------------------------------------
+// NC: through the read-only path; a kernel that also writes the array between
+// grid barriers (the persistent batch step) reads it plainly
+template <bool NC, class T> __device__ __forceinline__ T ldro(const T* p) {
+    if constexpr (NC) return __ldg(p); else return *p;
+}
+
+template <int S, class R>
+__device__ __forceinline__ void yee_rk(R x, R av, R cv, R d, R* out, R* acc, R* cmp, int e) {
+    if constexpr (is_mixed<R>::value) {
+        if (S == 0) { out[e] = fma_rn(d, 0.5f, x); acc[e] = mul_rn(d, 1.f / 6.f); }
+        else if (S == 1) { out[e] = fma_rn(d, 0.5f, x); acc[e] = fma_rn(d, 1.f / 3.f, av); }
+        else if (S == 2) { out[e] = x + d; acc[e] = fma_rn(d, 1.f / 3.f, av); }
+        else {
+            float sum, err;
+            two_sum(x, fma_rn(d, 1.f / 6.f, av) + cv, sum, err);
+            acc[e] = sum;
+            cmp[e] = err;
+        }
+    } else {
+        if (S == 0) { out[e] = fma_rn(d, 0.5, x); acc[e] = fma_rn(d, kInv6, x); }
+        else if (S == 1) { out[e] = fma_rn(d, 0.5, x); acc[e] = fma_rn(d, kInv3, av); }
+        else if (S == 2) { out[e] = x + d; acc[e] = fma_rn(d, kInv3, av); }
+        else { acc[e] = fma_rn(d, kInv6, av); }
+    }
+}
+
+// E edges of the 256 (j, k) vertices bx of vertex plane by; FROMP: dP/dt
+// sources; UNI: every edge has class uc, of four material cells
+template <int S, class R, bool FROMP, bool UNI, bool NC = true>
+__device__ __forceinline__ void yee_E_body(const Params& P, const StageIOT<R>& io, const EmCls<R>* __restrict__ cls_g, int ncls,
+                                           const EmCls<R>& uc, int bx, int by, EmCls<R>* cl) {
+    if constexpr (!UNI) {
+        for (int q = threadIdx.x; q < ncls; q += blockDim.x) cl[q] = cls_g[q];
+        __syncthreads();
+    }
+    const int nx = P.nx, ny = P.ny, nz = P.nz;
+    const int t = bx * blockDim.x + threadIdx.x;
+    if (t >= (ny + 1) * (nz + 1)) return;
+    const int i = by;
+    const int j = t / (nz + 1), k = t - (t / (nz + 1)) * (nz + 1);
+    const bool ox = i < nx, oy = j < ny, oz = k < nz;
+    // the wrapped cell at the vertex and its lower neighbours
+    const int iw = ox ? i : 0, jw = oy ? j : 0, kw = oz ? k : 0;
+    const int im = iw == 0 ? nx - 1 : iw - 1, jm = jw == 0 ? ny - 1 : jw - 1, km = kw == 0 ? nz - 1 : kw - 1;
+    const int e[3] = {(i * (ny + 1) + j) * (nz + 1) + k, (i * ny + j) * (nz + 1) + k, (i * (ny + 1) + j) * nz + k};
+    const bool on[3] = {ox, oy, oz};
+    R rx, ry, rz;
+    if constexpr (is_mixed<R>::value) { rx = P.f.rdx; ry = P.f.rdy; rz = P.f.rdz; }
+    else { rx = P.rdx; ry = P.rdy; rz = P.rdz; }
+    const R z = R(0.);
+    const int rw = iw * ny + jw, rjm = iw * ny + jm, rim = im * ny + jw, rijm = im * ny + jm;      // (i, j) rows of cell arrays
+    const int yw = iw * (ny + 1) + jw, yim = im * (ny + 1) + jw;                                    // and of Hy
+    const R* const Hx = io.H_in.c[0];
+    const R* const Hy = io.H_in.c[1];
+    const R* const Hz = io.H_in.c[2];
+    const R hxb = ldro<NC>(Hx + rw * nz + kw), hxj = ldro<NC>(Hx + rjm * nz + kw), hxk = ldro<NC>(Hx + rw * nz + km);
+    const R hyb = ldro<NC>(Hy + yw * nz + kw), hyi = ldro<NC>(Hy + yim * nz + kw), hyk = ldro<NC>(Hy + yw * nz + km);
+    const R hzb = ldro<NC>(Hz + rw * (nz + 1) + kw), hzi = ldro<NC>(Hz + rim * (nz + 1) + kw), hzj = ldro<NC>(Hz + rjm * (nz + 1) + kw);
+    R self[3], x[3], av[3], cv[3], qv[3][4];
+    int kc[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        self[c] = x[c] = av[c] = cv[c] = z;
+        kc[c] = 0;
+        if (on[c]) {
+            self[c] = x[c] = ldro<NC>(io.E_in.c[c] + e[c]);
+            if (S > 0) { x[c] = ldro<NC>(io.E_x.c[c] + e[c]); av[c] = io.E_acc.c[c][e[c]]; }
+            if constexpr (is_mixed<R>::value) { if (S == 3) cv[c] = io.E_cmp.c[c][e[c]]; }
+            if constexpr (!UNI) kc[c] = ldro<NC>(io.ecls[c] + e[c]);
+        }
+    }
+    if constexpr (FROMP) {
+        // the four cells of each edge, in the order of EmCls::mask's bits
+        const int c00 = rw * nz, c0m = rjm * nz, cm0 = rim * nz, cmm = rijm * nz;
+        const R* q0 = io.q_in.c[0];
+        const R* q1 = io.q_in.c[1];
+        const R* q2 = io.q_in.c[2];
+        qv[0][0] = ldro<NC>(q0 + c0m + km); qv[0][1] = ldro<NC>(q0 + c0m + kw); qv[0][2] = ldro<NC>(q0 + c00 + km); qv[0][3] = ldro<NC>(q0 + c00 + kw);
+        qv[1][0] = ldro<NC>(q1 + cm0 + km); qv[1][1] = ldro<NC>(q1 + cm0 + kw); qv[1][2] = ldro<NC>(q1 + c00 + km); qv[1][3] = ldro<NC>(q1 + c00 + kw);
+        qv[2][0] = ldro<NC>(q2 + cmm + kw); qv[2][1] = ldro<NC>(q2 + cm0 + kw); qv[2][2] = ldro<NC>(q2 + c0m + kw); qv[2][3] = ldro<NC>(q2 + c00 + kw);
+    }
+    const bool yb = (j == 0 || j == ny) && !P.per_y, zb = (k == 0 || k == nz) && !P.per_z, xb = (i == 0 || i == nx) && !P.per_x;
+    const bool bnd[3] = {yb || zb, xb || zb, xb || yb};
+    const R curl[3] = {fma_rn(hzb - hzj, ry, -mul_rn(hyb - hyk, rz)), fma_rn(hxb - hxk, rz, -mul_rn(hzb - hzi, rx)),
+                       fma_rn(hyb - hyi, rx, -mul_rn(hxb - hxj, ry))};
+    R jf[3] = {z, z, z};
+    if (P.jf_on && ((km >= P.jf_k0 && km <= P.jf_k1) || (kw >= P.jf_k0 && kw <= P.jf_k1))) {
+        const R a = R(stage_drive(io, S).jf);
+        const int c = P.jf_comp;
+        const int xa = c == 0 ? iw : im, ya = c == 1 ? jw : jm, za = c == 2 ? kw : km;     // the lower cell across the edge
+        R sum = z;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            // the two directions across the edge in the order x, y, z; bit 1 of q steps the first, bit 0 the second
+            const bool b1 = (q >> 1) & 1, b0 = q & 1;
+            const int cx = c == 0 ? iw : (b1 ? iw : xa);
+            const int cy = c == 1 ? jw : ((c == 0 ? b1 : b0) ? jw : ya);
+            const int cz = c == 2 ? kw : (b0 ? kw : za);
+            sum = sum + jf_cell(P, io, a, c, cx, cy, cz);
+        }
+        sum = mul_rn(sum, R(0.25));
+        if (c == 0) jf[0] = sum; else if (c == 1) jf[1] = sum; else jf[2] = sum;
+    }
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        if (!on[c]) continue;
+        const EmCls<R>& ec = UNI ? uc : cl[kc[c]];
+        R rhs = fma_rn(-ec.cond, self[c], curl[c] - jf[c]);
+        if constexpr (FROMP) {
+            const uint32_t mask = UNI ? 15u : ec.mask;
+            R sum = z;
+#pragma unroll
+            for (int q = 0; q < 4; q++) sum = sum + (((mask >> q) & 1u) ? qv[c][q] : z);
+            rhs = fma_rn(-sum, ec.rpc, rhs);
+        }
+        yee_rk<S>(x[c], av[c], cv[c], bnd[c] ? z : mul_rn(ec.coef, rhs), io.E_out.c[c], io.E_acc.c[c], io.E_cmp.c[c], e[c]);
+    }
+}
+
+// H faces of the same vertices; FROMM: dM/dt sources
+template <int S, class R, bool FROMM, bool NC = true>
+__device__ __forceinline__ void yee_H_body(const Params& P, const StageIOT<R>& io, int nmat, int bx, int by, R* sMs) {
+    if constexpr (FROMM) {
+        // Ms of a ferromagnetic id, 0 otherwise
+        for (int q = threadIdx.x; q <= nmat; q += blockDim.x) sMs[q] = (q > 0 && (io.mats[q - 1].flags & MF_FM)) ? io.mats[q - 1].Ms : R(0.);
+        __syncthreads();
+    }
+    const int nx = P.nx, ny = P.ny, nz = P.nz;
+    const int t = bx * blockDim.x + threadIdx.x;
+    if (t >= (ny + 1) * (nz + 1)) return;
+    const int i = by;
+    const int j = t / (nz + 1), k = t - (t / (nz + 1)) * (nz + 1);
+    const bool ox = i < nx, oy = j < ny, oz = k < nz;
+    const int ex = (i * (ny + 1) + j) * (nz + 1) + k, ey = (i * ny + j) * (nz + 1) + k, ez = (i * (ny + 1) + j) * nz + k;
+    const bool on[3] = {oy && oz, ox && oz, ox && oy};
+    const int e[3] = {(i * ny + j) * nz + k, ez, ey};
+    R rx, ry, rz, mdt;
+    if constexpr (is_mixed<R>::value) { rx = P.f.rdx; ry = P.f.rdy; rz = P.f.rdz; mdt = P.f.mdt_mu0; }
+    else { rx = P.rdx; ry = P.rdy; rz = P.rdz; mdt = P.mdt_mu0; }
+    const R z = R(0.);
+    const R* const Ex = io.E_in.c[0];
+    const R* const Ey = io.E_in.c[1];
+    const R* const Ez = io.E_in.c[2];
+    const R s0 = ox ? ldro<NC>(Ex + ex) : z, s1 = oy ? ldro<NC>(Ey + ey) : z, s2 = oz ? ldro<NC>(Ez + ez) : z;
+    R n[6] = {z, z, z, z, z, z};
+    if (on[0]) { n[0] = ldro<NC>(Ez + ez + nz); n[1] = ldro<NC>(Ey + ey + 1); }
+    if (on[1]) { n[2] = ldro<NC>(Ex + ex + 1); n[3] = ldro<NC>(Ez + ez + (ny + 1) * nz); }
+    if (on[2]) { n[4] = ldro<NC>(Ey + ey + ny * (nz + 1)); n[5] = ldro<NC>(Ex + ex + nz + 1); }
+    R x[3] = {z, z, z}, av[3] = {z, z, z}, cv[3] = {z, z, z}, dms[3] = {z, z, z};
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        if (!on[c]) continue;
+        x[c] = ldro<NC>(io.H_x.c[c] + e[c]);
+        if (S > 0) av[c] = io.H_acc.c[c][e[c]];
+        if constexpr (is_mixed<R>::value) { if (S == 3) cv[c] = io.H_cmp.c[c][e[c]]; }
+    }
+    if constexpr (FROMM) {
+        // Ms dm of the two face cells over the number that are magnetic
+        // (EMdynamic_solver.cpp:2300-2306); at an open end both are the end cell
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            if (!on[c]) continue;
+            int a, b;
+            if (c == 0) {
+                const int lo = i == 0 ? (P.per_x ? nx - 1 : 0) : i - 1, hi = ox ? i : (P.per_x ? 0 : nx - 1);
+                a = (lo * ny + j) * nz + k; b = (hi * ny + j) * nz + k;
+            } else if (c == 1) {
+                const int lo = j == 0 ? (P.per_y ? ny - 1 : 0) : j - 1, hi = oy ? j : (P.per_y ? 0 : ny - 1);
+                a = (i * ny + lo) * nz + k; b = (i * ny + hi) * nz + k;
+            } else {
+                const int lo = k == 0 ? (P.per_z ? nz - 1 : 0) : k - 1, hi = oz ? k : (P.per_z ? 0 : nz - 1);
+                a = (i * ny + j) * nz + lo; b = (i * ny + j) * nz + hi;
+            }
+            const R da = ldro<NC>(io.dm.c[c] + a), db = ldro<NC>(io.dm.c[c] + b);
+            const R ma = sMs[ldro<NC>(io.mid + a)], mb = sMs[ldro<NC>(io.mid + b)];
+            R sum = z;
+            if (ma != z) sum = mul_rn(da, ma);
+            if (mb != z) sum = fma_rn(db, mb, sum);
+            dms[c] = (ma != z && mb != z) ? mul_rn(sum, R(0.5)) : sum;
+        }
+    }
+    const R curl[3] = {fma_rn(n[0] - s2, ry, -mul_rn(n[1] - s1, rz)), fma_rn(n[2] - s0, rz, -mul_rn(n[3] - s2, rx)),
+                       fma_rn(n[4] - s1, rx, -mul_rn(n[5] - s0, ry))};
+#pragma unroll
+    for (int c = 0; c < 3; c++)
+        if (on[c]) yee_rk<S>(x[c], av[c], cv[c], fma_rn(mdt, curl[c], -dms[c]), io.H_out.c[c], io.H_acc.c[c], io.H_cmp.c[c], e[c]);
+}
+
+// Blocks of 256 threads per SM the registers allow: as many as keep a thread's
+// loads (up to 30 before its first use) in registers.  Both kernels are bound
+// by memory and the issue of the loads together (us per launch, 128^3
+// ferroelectric grid, k_em_fused before: FP64 152 -> E 64 + H 31, FP32 102 ->
+// E 36 + H 20; the two run on streams of their own).  A march along x that
+// kept the planes' values in registers was no faster (FP64 114, FP32 81 for
+// the pair in one kernel): it carries three planes and waits for each.
+template <class R, bool FROMP> constexpr int kYeeEBlocks = is_mixed<R>::value ? 4 : (FROMP ? 2 : 3);
+template <class R, bool FROMM> constexpr int kYeeHBlocks = is_mixed<R>::value ? (FROMM ? 6 : 8) : (FROMM ? 4 : 5);
+template <int S, class R, bool FROMP, bool UNI>
+__global__ void __launch_bounds__(256, (kYeeEBlocks<R, FROMP>))
+    k_yee_E(const __grid_constant__ Params P, const __grid_constant__ StageIOT<R> io, const EmCls<R>* __restrict__ cls_g, int ncls,
+            const __grid_constant__ EmCls<R> uc) {
+    __shared__ EmCls<R> cl[UNI ? 1 : kEmMaxCls];
+    yee_E_body<S, R, FROMP, UNI>(P, io, cls_g, ncls, uc, blockIdx.x, blockIdx.y, cl);
+}
+template <int S, class R, bool FROMM>
+__global__ void __launch_bounds__(256, (kYeeHBlocks<R, FROMM>))
+    k_yee_H(const __grid_constant__ Params P, const __grid_constant__ StageIOT<R> io, int nmat) {
+    __shared__ R sMs[kMaxMat + 1];
+    yee_H_body<S, R, FROMM>(P, io, nmat, blockIdx.x, blockIdx.y, sMs);
+}
+
+// runs the two kernels cover
+__host__ __device__ inline bool yee_path(const Params& P) { return P.em_cls && !P.drude && !P.spin && !P.afm; }
 
 // Drude polarisation current, per cell: dJp_n = (e0 wp_n^2 E_cell c_n -
 // Jp_n / tau_n) dt for the three poles (get_dJp_RK{1..4},

@@ -74,9 +74,9 @@ struct gf_engine {
     cudaStream_t stream = nullptr;
     // branch streams of a stage (LLG, TDGL, Maxwell) and their fork / join
     // events; the elastic chain and the static solves stay on `stream`
-    cudaStream_t side[3] = {nullptr, nullptr, nullptr};
+    cudaStream_t side[4] = {nullptr, nullptr, nullptr, nullptr};
     bool prio_nodes = false;               // the streams have unequal priorities (kept by the step graph)
-    cudaEvent_t bev[6] = {};
+    cudaEvent_t bev[7] = {};
     std::string err;
 
     // bookkeeping
@@ -123,6 +123,10 @@ struct gf_engine {
     int el_nmat = 0;                   // materials staged by k_elastic_tile
     size_t el_smem = 0;                // its dynamic shared memory
     bool el_cubic = false;             // every material has the cubic stiffness pattern
+    // the only class of the E edges, of four material cells
+    bool em_uni = false;
+    EmCls<double> em_uc = {};
+    EmCls<float> em_uc_f = {};
     // every cell is material 1, whose constants the kernels of such runs take by value
     bool uni = false;
     DevMat um = {};
@@ -1097,15 +1101,40 @@ int enqueue_fe(gf_engine* eng, const StageIOT<R>& io, cudaStream_t st) {
     return GF_OK;
 }
 
-// Maxwell kernels of stage S on stream st: the Yee update, then the plane
-// source, the Mur boundaries, PEC and the Drude currents, in that order
+template <class R>
+const EmCls<R>& em_ucls(const gf_engine* eng) {
+    if constexpr (is_mixed<R>::value) return eng->em_uc_f; else return eng->em_uc;
+}
+// H faces of stage S on stream st (runs k_yee_E / k_yee_H cover)
 template <int S, class R>
-int enqueue_em(gf_engine* eng, const StageIOT<R>& io, cudaStream_t st) {
+int enqueue_yee_H(gf_engine* eng, const StageIOT<R>& io, cudaStream_t st) {
+    const Params& P = eng->P;
+    const dim3 g(blocks_for((long)(P.ny + 1) * (P.nz + 1), kThreads), (unsigned)(P.nx + 1));
+    const int nm = (int)eng->deck.mats.size();
+    if (P.em_fromM) GF_CU(klaunch(eng, "k_yee_H", k_yee_H<S, R, true>, g, dim3(kThreads), 0, st, P, io, nm));
+    else GF_CU(klaunch(eng, "k_yee_H", k_yee_H<S, R, false>, g, dim3(kThreads), 0, st, P, io, nm));
+    return GF_OK;
+}
+
+// Maxwell kernels of stage S on stream st: the Yee update (with_H: of the H
+// faces too), then the plane source, the Mur boundaries, PEC and the Drude
+// currents, in that order
+template <int S, class R>
+int enqueue_em(gf_engine* eng, const StageIOT<R>& io, cudaStream_t st, bool with_H) {
     const Params& P = eng->P;
     const long nx = P.nx, ny = P.ny, nz = P.nz;
-    GF_CU(klaunch<true>(eng, "k_em_fused", k_em_fused<S, R>, dim3(blocks_for((ny + 1) * (nz + 1), kThreads), (unsigned)(nx + 1)),
-                  dim3(kThreads), 0, st, P, io, (int)eng->deck.mats.size(),
-                  static_cast<const EmCls<R>*>(eng->em_cls_tab), eng->em_ncls));
+    const dim3 g(blocks_for((ny + 1) * (nz + 1), kThreads), (unsigned)(nx + 1));
+    const EmCls<R>* cls = static_cast<const EmCls<R>*>(eng->em_cls_tab);
+    if (!yee_path(P)) {
+        GF_CU(klaunch<true>(eng, "k_em_fused", k_em_fused<S, R>, g, dim3(kThreads), 0, st, P, io, (int)eng->deck.mats.size(), cls, eng->em_ncls));
+    } else {
+        auto E = [&](auto k) { return klaunch<true>(eng, "k_yee_E", k, g, dim3(kThreads), 0, st, P, io, cls, eng->em_ncls, em_ucls<R>(eng)); };
+        if (P.em_fromP && eng->em_uni) GF_CU(E(k_yee_E<S, R, true, true>));
+        else if (P.em_fromP) GF_CU(E(k_yee_E<S, R, true, false>));
+        else if (eng->em_uni) GF_CU(E(k_yee_E<S, R, false, true>));
+        else GF_CU(E(k_yee_E<S, R, false, false>));
+        if (with_H) GF_TRY((enqueue_yee_H<S, R>(eng, io, st)));
+    }
     if (P.planeEM) GF_CU(klaunch(eng, "k_em_plane", k_em_plane<S, R>, dim3(blocks_for(nx * ny, kThreads)), dim3(kThreads), 0, st, P, io));
     if (!P.per_x) GF_CU(klaunch(eng, "k_em_mur_x", k_em_mur<S, 0, R>, dim3(blocks_for(ny * (nz + 1) + (ny + 1) * nz, kThreads)), dim3(kThreads), 0, st, P, io));
     if (!P.per_y) GF_CU(klaunch(eng, "k_em_mur_y", k_em_mur<S, 1, R>, dim3(blocks_for(nx * (nz + 1) + (nx + 1) * nz, kThreads)), dim3(kThreads), 0, st, P, io));
@@ -1138,17 +1167,26 @@ int enqueue_stage(gf_engine* eng, int parity) {
     const bool par = !eng->profiling && groups >= 2;
     auto rec = [&](cudaEvent_t e, cudaStream_t s_) { return par ? cudaEventRecord(e, s_) : cudaSuccess; };
     auto wait_ = [&](cudaStream_t s_, cudaEvent_t e, unsigned) { return par ? cudaStreamWaitEvent(s_, e, 0) : cudaSuccess; };
-    cudaStream_t s_llg = par ? eng->side[0] : st, s_fe = par ? eng->side[1] : st, s_em = par ? eng->side[2] : st;
+    cudaStream_t s_llg = par ? eng->side[0] : st, s_fe = par ? eng->side[1] : st, s_em = par ? eng->side[2] : st, s_emh = par ? eng->side[3] : st;
     cudaEvent_t ev_start = eng->bev[0], ev_pre = eng->bev[1], ev_tile = eng->bev[2];
-    cudaEvent_t ev_llg = eng->bev[3], ev_fe = eng->bev[4], ev_em = eng->bev[5];
+    cudaEvent_t ev_llg = eng->bev[3], ev_fe = eng->bev[4], ev_em = eng->bev[5], ev_emh = eng->bev[6];
     const bool mag = P.fm || P.afm;
-    const bool em_after_llg = P.em && mag && (P.em_fromM || P.spin);
+    // the H faces as a kernel beside the E edges' (PEC clears the step-start E
+    // that the H faces read at stage 1: it then runs after them, in one chain)
+    const bool em_split = P.em && yee_path(P) && !P.pec;
+    const bool em_after_llg = P.em && mag && (P.em_fromM || P.spin) && !em_split;
+    const bool h_after_llg = em_split && mag && P.em_fromM;
     const bool em_after_fe = P.em && P.fe && P.pec;
     GF_CU(rec(ev_start, st));
     if (P.em && !em_after_llg && !em_after_fe) {
         GF_CU(wait_(s_em, ev_start, 0));
-        GF_TRY((enqueue_em<S, R>(eng, io, s_em)));
+        GF_TRY((enqueue_em<S, R>(eng, io, s_em, !em_split)));
         GF_CU(rec(ev_em, s_em));
+    }
+    if (em_split && !h_after_llg) {
+        GF_CU(wait_(s_emh, ev_start, 0));
+        GF_TRY((enqueue_yee_H<S, R>(eng, io, s_emh)));
+        GF_CU(rec(ev_emh, s_emh));
     }
     if (P.flexo)
         GF_CU(klaunch(eng, "k_flexo_prep", k_flexo_prep<R>, dim3(blocks_for((long)P.ny * P.nz, kThreads), (unsigned)P.nx),
@@ -1187,8 +1225,13 @@ int enqueue_stage(gf_engine* eng, int parity) {
     if (P.em && (em_after_llg || em_after_fe)) {
         if (em_after_llg) GF_CU(wait_(s_em, ev_llg, 0));
         if (em_after_fe) GF_CU(wait_(s_em, ev_fe, 0));
-        GF_TRY((enqueue_em<S, R>(eng, io, s_em)));
+        GF_TRY((enqueue_em<S, R>(eng, io, s_em, !em_split)));
         GF_CU(rec(ev_em, s_em));
+    }
+    if (h_after_llg) {
+        GF_CU(wait_(s_emh, ev_llg, 0));
+        GF_TRY((enqueue_yee_H<S, R>(eng, io, s_emh)));
+        GF_CU(rec(ev_emh, s_emh));
     }
     if (P.elastic) {
         // the mixed form's RK kernel updates two cells per thread
@@ -1201,6 +1244,7 @@ int enqueue_stage(gf_engine* eng, int parity) {
     if (mag) GF_CU(wait_(st, ev_llg, 0));
     if (P.fe) GF_CU(wait_(st, ev_fe, 0));
     if (P.em) GF_CU(wait_(st, ev_em, 0));
+    if (em_split) GF_CU(wait_(st, ev_emh, 0));
     if (eng->demag_per_stage) {
         // static field of the new stage state (main.cpp:299-306, 476-483)
         if constexpr (is_mixed<R>::value) GF_TRY(demag_solve_f32(eng, io.m_out, io.a1_out, io.a2_out, true, io.msrc != nullptr));
@@ -1784,6 +1828,7 @@ EmCls<R> em_class(const Deck& d, const unsigned ids[4], R dt_e0) {
     c.coef = dt_e0 / er;
     c.cond = cond / R(4.);
     c.pc = pc;
+    c.rpc = R(1.) / pc;
     c.mask = mask;
     c.pad_ = 0;
     return c;
@@ -1862,6 +1907,13 @@ int setup_em_classes(gf_engine* eng) {
         GF_CU(cudaMemcpy(eng->ecls[C], cls[C].data(), cls[C].size(), cudaMemcpyHostToDevice));
     }
     eng->em_ncls = (int)nk;
+    {
+        unsigned ids[4];
+        ids_of(keys[0], ids);
+        eng->em_uc = em_class<double>(d, ids, P.dt_e0);
+        eng->em_uc_f = em_class<float>(d, ids, P.f.dt_e0);
+        eng->em_uni = nk == 1 && eng->em_uc.mask == 15u;
+    }
     P.em_cls = 1;
     return GF_OK;
 }
@@ -1967,6 +2019,7 @@ int create_from(gf_engine* eng, const std::string& dir, int device, int precisio
         GF_CU(cudaStreamCreateWithPriority(&eng->side[0], cudaStreamNonBlocking, pl));
         GF_CU(cudaStreamCreateWithPriority(&eng->side[1], cudaStreamNonBlocking, pf));
         GF_CU(cudaStreamCreateWithPriority(&eng->side[2], cudaStreamNonBlocking, pe));
+        GF_CU(cudaStreamCreateWithPriority(&eng->side[3], cudaStreamNonBlocking, pe));
     }
     const long n = P.n;
     if (eng->mixed) {
@@ -3611,8 +3664,11 @@ void batch_items(const gf_batch* b, const std::vector<int>& ch, std::vector<Batc
         }
         if (P.em) {
             const int gx = (int)blocks_for((ny + 1) * (nz + 1), kThreads);
-            for (int y = 0; y <= P.nx; y++)
-                for (int x = 0; x < gx; x++) Ae.push_back({in, BK_EM, x, y, 0});
+            // E edges and H faces as items of their own where the engine has
+            // two kernels for them
+            for (int z = 0; z < (yee_path(P) ? 2 : 1); z++)
+                for (int y = 0; y <= P.nx; y++)
+                    for (int x = 0; x < gx; x++) Ae.push_back({in, BK_EM, x, y, z});
             std::vector<BatchItem>* ph[3] = {&B, &C, &D};
             int q = 0;
             if (!P.per_x) { for (int x = 0; x < (int)blocks_for(ny * (nz + 1) + (ny + 1) * nz, kThreads); x++) ph[q]->push_back({in, BK_MUR_X, x, 0, 0}); q++; }

@@ -151,3 +151,35 @@ def test_tdgl_of_one_material_equals_two_alike(gf, shape, elastic, precision):
     g = dataclasses.replace(d, materials=[d.materials[0]] * 2)
     g.struct = np.random.default_rng(37).integers(1, 3, shape).astype(np.uint8)
     _same(_run(gf, d, precision), _run(gf, g, precision), TOL[precision])
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("name", ["fe_z", "fe_x_type1", "fe_y_type6", "open", "periodic_z", "fm_sources", "both", "vacuum_film", "one_cell"])
+def test_yee_update_equals_the_general_one(gf, name, precision):
+    D = gf.decks
+    if name == "fm_sources":
+        d = _me(gf, 6, 9, 12, 5, 4)
+    elif name == "both":
+        d = _scattered(gf, 6, 8, 7, [D.pto(), D.yig(1e-2)], 5, em_fromM=True, em_back_M=True)
+    elif name == "vacuum_film":
+        d = _fe(gf, 5, 8, 8, layers=[(3, 0), (3, 1), (2, 0)])
+    elif name == "one_cell":
+        d = _fe(gf, 1, 1, 5, elastic=False, elasto_back=False, elasto_on=False)
+    else:
+        d = _fe(gf, 6, 11, 9)
+        d.jf_lo, d.jf_hi = (1, 0, 2), (4, 8, 5)
+        if name == "fe_x_type1":
+            d.jf_comp, d.jf_type, d.jf_freq = "x", 1, 1e15
+        elif name == "fe_y_type6":
+            d.jf_comp, d.jf_type, d.jf_freq, d.jf_sigma = "y", 6, 1e15, 2e-17
+        elif name == "open":
+            d.periodic = (False, False, False)
+        elif name == "periodic_z":
+            d = dataclasses.replace(d, ny=9, jf_hi=(4, 8, 8), jf_lo=(0, 0, 7), periodic=(True, True, True), elastic=False,
+                                    elasto_back=False, elasto_on=False)
+            d.p0 = d.q0 = None
+    d = _moving(d, 19)
+    # a material with a Drude pole that no cell has: no current flows
+    pole = dataclasses.replace(D.ggg(), drude=((1.0, 1e15, 1e-14), (0.0, 0.0, 1.0), (0.0, 0.0, 1.0)))
+    g = dataclasses.replace(d, materials=list(d.materials) + [pole])
+    _same(_run(gf, d, precision), _run(gf, g, precision), TOL[precision])
