@@ -28,7 +28,7 @@
 #pragma once
 
 #include "gf_state.cuh"
-#include "gf_elastic.cuh"
+#include "gf_column.cuh"
 
 namespace gf {
 
@@ -58,16 +58,16 @@ template <class R> __device__ inline R dot3(V3<R> a, V3<R> b) { return a.x * b.x
 template <class R> __device__ inline V3<R> ld3(const F3T<R>& f, int c) { return mk3<R>(f.c[0][c], f.c[1][c], f.c[2][c]); }
 template <class R> __device__ inline void st3(const F3T<R>& f, int c, V3<R> v) { f.c[0][c] = v.x; f.c[1][c] = v.y; f.c[2][c] = v.z; }
 
-// neighbour cells with periodic wrap and the exchange weight A_cf / dx_f^2
-// of each face (0 on ferromagnetic surfaces and non-periodic boundaries)
+// Neighbour cells with periodic wrap (adj_cells: their fields can be loaded
+// before their ids are known) and the exchange weight A_cf / dx_f^2 of each
+// face (0 on ferromagnetic surfaces and non-periodic boundaries)
 template <class R>
 struct AdjNbr {
     int nb[6];
     R w[6];
 };
 template <class R>
-__device__ inline void adj_neighbours(const Params& P, const uint8_t* mid, const AdjMatT<R>* am, const R* aij, int nmat,
-                                      int i, int j, int k, uint8_t id, AdjNbr<R>& n) {
+__device__ inline void adj_cells(const Params& P, int i, int j, int k, AdjNbr<R>& n) {
     const int nx = P.nx, ny = P.ny, nz = P.nz;
     const int ib = (i == 0) ? nx - 1 : i - 1, iF = (i == nx - 1) ? 0 : i + 1;
     const int jb = (j == 0) ? ny - 1 : j - 1, jF = (j == ny - 1) ? 0 : j + 1;
@@ -75,6 +75,11 @@ __device__ inline void adj_neighbours(const Params& P, const uint8_t* mid, const
     n.nb[0] = (ib * ny + j) * nz + k; n.nb[1] = (iF * ny + j) * nz + k;
     n.nb[2] = (i * ny + jb) * nz + k; n.nb[3] = (i * ny + jF) * nz + k;
     n.nb[4] = (i * ny + j) * nz + kb; n.nb[5] = (i * ny + j) * nz + kF;
+}
+template <class R>
+__device__ inline void adj_weights(const Params& P, const uint8_t* mid, const AdjMatT<R>* am, const R* aij, int nmat,
+                                   int i, int j, int k, uint8_t id, AdjNbr<R>& n) {
+    const int nx = P.nx, ny = P.ny, nz = P.nz;
     const bool edge[6] = {i == 0 && !P.per_x, i == nx - 1 && !P.per_x, j == 0 && !P.per_y,
                           j == ny - 1 && !P.per_y, k == 0 && !P.per_z, k == nz - 1 && !P.per_z};
     const R r2[3] = {R(P.rdx * P.rdx), R(P.rdy * P.rdy), R(P.rdz * P.rdz)};
@@ -93,7 +98,7 @@ __device__ inline void adj_neighbours(const Params& P, const uint8_t* mid, const
 // value carries a compensation word xc: stage 3 forms x + (acc + k/6) + xc
 // by an error-free sum (the mixed engine's compensated RK update).
 template <int S, class R>
-__global__ void __launch_bounds__(256) k_adj_eval(Params P, const uint8_t* __restrict__ mid, const AdjMatT<R>* __restrict__ am,
+__global__ void __launch_bounds__(256, is_mixed<R>::value ? 4 : 3) k_adj_eval(Params P, const uint8_t* __restrict__ mid, const AdjMatT<R>* __restrict__ am,
                                                   const R* __restrict__ aij, int nmat, F3T<R> y, F3T<R> hd,
                                                   const R* __restrict__ alpha, V3<R> hext, F3T<R> hs, F3T<R> x, F3T<R> xc,
                                                   F3T<R> acc, F3T<R> ynext, C6T<R> str) {
@@ -101,20 +106,36 @@ __global__ void __launch_bounds__(256) k_adj_eval(Params P, const uint8_t* __res
     if (c >= P.n) return;
     const int nyz = P.ny * P.nz;
     const int i = c / nyz, j = (c - i * nyz) / P.nz, k = c - i * nyz - j * P.nz;
+    // every operand that does not depend on the ids is loaded before the first
+    // use, so that the loads fly together (256x256x32 FP32 film, ncu: 74 us per
+    // launch with the loads where they were used)
     const uint8_t id = mid[c];
+    AdjNbr<R> n;
+    adj_cells(P, i, j, k, n);
+    const V3<R> m = ld3(y, c);
+    V3<R> mn[6];
+#pragma unroll
+    for (int f = 0; f < 6; f++) mn[f] = ld3(y, n.nb[f]);
+    V3<R> H = ld3(hd, c);
+    R e[6] = {R(0), R(0), R(0), R(0), R(0), R(0)};
+    if (str.c[0]) {
+#pragma unroll
+        for (int q = 0; q < 6; q++) e[q] = str.c[q][c];
+    }
+    const V3<R> x0 = ld3(x, c);
+    V3<R> a0 = mk3<R>(R(0), R(0), R(0)), c0 = a0;
+    if (S > 0) a0 = ld3(acc, c);
+    if constexpr (is_mixed<R>::value) { if (S == 3) c0 = ld3(xc, c); }
+    const R al = alpha[c];
     V3<R> kk = mk3<R>(R(0), R(0), R(0));
     if (id != 0 && am[id - 1].fm) {
         const AdjMatT<R>& mt = am[id - 1];
-        AdjNbr<R> n;
-        adj_neighbours(P, mid, am, aij, nmat, i, j, k, id, n);
-        const V3<R> m = ld3(y, c);
+        adj_weights(P, mid, am, aij, nmat, i, j, k, id, n);
         V3<R> hex = mk3<R>(R(0), R(0), R(0));
 #pragma unroll
         for (int f = 0; f < 6; f++) {
-            const V3<R> mf = ld3(y, n.nb[f]);
-            hex.x += n.w[f] * (mf.x - m.x); hex.y += n.w[f] * (mf.y - m.y); hex.z += n.w[f] * (mf.z - m.z);
+            hex.x += n.w[f] * (mn[f].x - m.x); hex.y += n.w[f] * (mn[f].y - m.y); hex.z += n.w[f] * (mn[f].z - m.z);
         }
-        V3<R> H = ld3(hd, c);
         H.x += mt.ex_coef * hex.x + hext.x; H.y += mt.ex_coef * hex.y + hext.y; H.z += mt.ex_coef * hex.z + hext.z;
         if (mt.aniso == 1) {
             H.x += R(-2) * (mt.K1c * (m.y * m.y + m.z * m.z) + mt.K2c * m.y * m.y * m.z * m.z) * m.x;
@@ -125,39 +146,37 @@ __global__ void __launch_bounds__(256) k_adj_eval(Params P, const uint8_t* __res
         }
         if (str.c[0]) {
             // magnetoelastic field of the stage strain (the engine's k_llg_fm)
-            const R exx = str.c[0][c], eyy = str.c[1][c], ezz = str.c[2][c];
-            const R eyz = str.c[3][c], exz = str.c[4][c], exy = str.c[5][c];
+            const R exx = e[0], eyy = e[1], ezz = e[2], eyz = e[3], exz = e[4], exy = e[5];
             H.x += R(-2) * (mt.B1c * exx * m.x + mt.B2c * (exy * m.y + exz * m.z));
             H.y += R(-2) * (mt.B1c * eyy * m.y + mt.B2c * (exy * m.x + eyz * m.z));
             H.z += R(-2) * (mt.B1c * ezz * m.z + mt.B2c * (exz * m.x + eyz * m.y));
         }
         st3(hs, c, H);
-        const R a = alpha[c];
-        const R c1 = -mt.gdt / (R(1) + a * a), c2 = a * c1;
+        const R c1 = -mt.gdt / (R(1) + al * al), c2 = al * c1;
         const V3<R> p = cross3(m, H), q = cross3(m, p);
         kk = mk3<R>(c1 * p.x + c2 * q.x, c1 * p.y + c2 * q.y, c1 * p.z + c2 * q.z);
     } else {
         st3(hs, c, mk3<R>(R(0), R(0), R(0)));
     }
-    const R kv[3] = {kk.x, kk.y, kk.z};
+    const R kv[3] = {kk.x, kk.y, kk.z}, xs[3] = {x0.x, x0.y, x0.z}, as[3] = {a0.x, a0.y, a0.z}, cs[3] = {c0.x, c0.y, c0.z};
 #pragma unroll
     for (int a = 0; a < 3; a++) {
-        const R xv = x.c[a][c];
+        const R xv = xs[a];
         if constexpr (is_mixed<R>::value) {
             if (S == 0) { acc.c[a][c] = kv[a] * (1.f / 6.f); ynext.c[a][c] = xv + kv[a] * 0.5f; }
-            else if (S == 1) { acc.c[a][c] = acc.c[a][c] + kv[a] * (1.f / 3.f); ynext.c[a][c] = xv + kv[a] * 0.5f; }
-            else if (S == 2) { acc.c[a][c] = acc.c[a][c] + kv[a] * (1.f / 3.f); ynext.c[a][c] = xv + kv[a]; }
+            else if (S == 1) { acc.c[a][c] = as[a] + kv[a] * (1.f / 3.f); ynext.c[a][c] = xv + kv[a] * 0.5f; }
+            else if (S == 2) { acc.c[a][c] = as[a] + kv[a] * (1.f / 3.f); ynext.c[a][c] = xv + kv[a]; }
             else {
                 float sum, err;
-                two_sum(xv, (acc.c[a][c] + kv[a] * (1.f / 6.f)) + xc.c[a][c], sum, err);
+                two_sum(xv, (as[a] + kv[a] * (1.f / 6.f)) + cs[a], sum, err);
                 x.c[a][c] = sum;
                 xc.c[a][c] = err;
             }
         } else {
-            if (S == 0) { acc.c[a][c] = kv[a] / 6.; ynext.c[a][c] = xv + kv[a] * 0.5; }
-            else if (S == 1) { acc.c[a][c] = acc.c[a][c] + kv[a] / 3.; ynext.c[a][c] = xv + kv[a] * 0.5; }
-            else if (S == 2) { acc.c[a][c] = acc.c[a][c] + kv[a] / 3.; ynext.c[a][c] = xv + kv[a]; }
-            else { x.c[a][c] = xv + (acc.c[a][c] + kv[a] / 6.); }
+            if (S == 0) { acc.c[a][c] = kv[a] * kInv6; ynext.c[a][c] = xv + kv[a] * 0.5; }
+            else if (S == 1) { acc.c[a][c] = as[a] + kv[a] * kInv3; ynext.c[a][c] = xv + kv[a] * 0.5; }
+            else if (S == 2) { acc.c[a][c] = as[a] + kv[a] * kInv3; ynext.c[a][c] = xv + kv[a]; }
+            else { x.c[a][c] = xv + (as[a] + kv[a] * kInv6); }
         }
     }
 }
@@ -294,159 +313,91 @@ __global__ void __launch_bounds__(256) k_adj_el_vjp(Params P, const uint8_t* __r
     }
 }
 
-// Pass 1 of the transposed stress stencil, per cell x: for each of its six
-// faces that is not stress-free, the face-stress cotangent
-// sbar = (fbar_lower - fbar_upper) / h (the face adds +sigma/h to the force
-// of the cell below it and -sigma/h to the one above), half of it to x's side
-// (sigma = mean of the two sides), through the rows of C_x to x's side
-// strain st (k_elastic_tile's side_rows: face normal and face shears from the
-// face's own gradient, the other components from x's face-gradient means,
-// engineering shears, minus e0).  Outputs per cell (27 x n, `to`):
-//   T[d][a] (9): cotangent of x's gradient du_a/dx_d on both of its d-faces
-//               (every mean (g_minus + g_plus)/2 or /4 enters both alike),
-//               plus the LLG strain's cotangent (the cell strain is the same
-//               means);
-//   O[f][a] (18): cotangent of the gradient on face f (2d: -d, 2d+1: +d) from
-//               x's own side of that face (normal and face shears).
-// The eigenstrain cotangent -st (x2 for shears) goes through the
-// magnetostriction e0_aa = 1.5 l100 (m_a^2 - 1/3), e0_ab = 1.5 l111 m_a m_b
-// into ybar_m (back: the run feeds the eigenstrain back).
-// With elastodynamics ybar_m is final here: the m group's RK combination
-// (adj_comb1 at stage s: lam_m, lamacc_m, u_m) follows in the same thread.
+// Transposed stress and strain stencils of a stage with the RK combination of
+// the u group (adj_comb1), in one march of col_march: the stress divergence is
+// a symmetric operator (f = sum over faces of D^T C D u with the cubic
+// material's c_a g_a + K_a per cell and face), so its transpose is the same
+// march over the force cotangent fbar.  What is not symmetric rides along: the
+// LLG strain's cotangent enters a cell's gradient cotangents through the same
+// gradient means (e_aa = T[a][a] / 2, e_ab = (T[a][b] + T[b][a]) / 4), i.e. as
+// EN = strbar_aa and ES = strbar_ab / 2; and the eigenstrain's cotangent is
+// formed from the sums of fbar's gradients,
+//   ebar_aa = (c11 T[a][a] + c12 (T[b][b] + T[c][c])) / 2,
+//   ebar_ab = c44 (T[a][b] + T[b][a]),
+// and goes through the magnetostriction e0_aa = 1.5 l100 (m_a^2 - 1/3),
+// e0_ab = 1.5 l111 m_a m_b into ybar_m (back: the run feeds the eigenstrain
+// back; k_adj_field_T then completes ybar_m).  The operands of a cell's
+// outputs are loaded at the start of its plane, so that they fly while the
+// plane is computed.
 template <class R>
-__global__ void __launch_bounds__(256) k_adj_el_p1(Params P, const uint8_t* __restrict__ mid, const DevMatT<R>* __restrict__ mats,
-                                                  F3T<R> fbar, C6T<R> strbar, F3T<R> m, F3T<R> ybar_m, int back, R* __restrict__ to,
-                                                  int s, F3T<R> lam_m, F3T<R> lamacc_m, F3T<R> u_m) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= P.n) return;
-    const long n = P.n;
-    R T[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}}, O[6][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}, {0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-    const uint8_t id = mid[c];
-    if (id != 0) {
-        const DevMatT<R>& mt = mats[id - 1];
-        const int nyz = P.ny * P.nz;
-        const int i = c / nyz, j = (c - i * nyz) / P.nz, k = c - i * nyz - j * P.nz;
-        const int pos[3] = {i, j, k}, nn[3] = {P.nx, P.ny, P.nz}, per[3] = {P.per_x, P.per_y, P.per_z};
-        const int stride[3] = {nyz, P.nz, 1};
-        const R rh[3] = {R(P.rdx), R(P.rdy), R(P.rdz)};
-        R d0b[6] = {0, 0, 0, 0, 0, 0};
-        const R fx[3] = {fbar.c[0][c], fbar.c[1][c], fbar.c[2][c]};
-        for (int D = 0; D < 3; D++) {
-            for (int side = 0; side < 2; side++) {
-                const bool edge = side == 0 ? pos[D] == 0 : pos[D] == nn[D] - 1;
-                if (edge && !per[D]) continue;
-                int q = pos[D] + (side == 0 ? -1 : 1);
-                q = q < 0 ? q + nn[D] : (q >= nn[D] ? q - nn[D] : q);
-                const int y = c + (q - pos[D]) * stride[D];
-                if (mid[y] == 0) continue;
-                const R fy_[3] = {fbar.c[0][y], fbar.c[1][y], fbar.c[2][y]};
-                R S_[3];
-#pragma unroll
-                for (int r = 0; r < 3; r++) {
-                    const R lo = side == 0 ? fy_[r] : fx[r], up = side == 0 ? fx[r] : fy_[r];
-                    S_[r] = R(0.5) * (lo - up) * rh[D];
-                }
-                R st[6];
-#pragma unroll
-                for (int qv = 0; qv < 6; qv++)
-                    st[qv] = mt.cij[face_row(D, 0)][qv] * S_[0] + mt.cij[face_row(D, 1)][qv] * S_[1]
-                             + mt.cij[face_row(D, 2)][qv] * S_[2];
-                R* o = O[2 * D + side];
-                if (D == 0) {
-                    o[0] += st[0]; o[2] += st[4]; o[1] += st[5];
-                    T[1][1] += R(0.5) * st[1]; T[2][2] += R(0.5) * st[2];
-                    T[2][1] += R(0.5) * st[3]; T[1][2] += R(0.5) * st[3];
-                    T[2][0] += R(0.5) * st[4]; T[1][0] += R(0.5) * st[5];
-                } else if (D == 1) {
-                    o[1] += st[1]; o[2] += st[3]; o[0] += st[5];
-                    T[0][0] += R(0.5) * st[0]; T[2][2] += R(0.5) * st[2];
-                    T[2][1] += R(0.5) * st[3];
-                    T[2][0] += R(0.5) * st[4]; T[0][2] += R(0.5) * st[4];
-                    T[0][1] += R(0.5) * st[5];
-                } else {
-                    o[2] += st[2]; o[1] += st[3]; o[0] += st[4];
-                    T[0][0] += R(0.5) * st[0]; T[1][1] += R(0.5) * st[1];
-                    T[1][2] += R(0.5) * st[3]; T[0][2] += R(0.5) * st[4];
-                    T[1][0] += R(0.5) * st[5]; T[0][1] += R(0.5) * st[5];
-                }
-                d0b[0] -= st[0]; d0b[1] -= st[1]; d0b[2] -= st[2];
-                d0b[3] -= R(2) * st[3]; d0b[4] -= R(2) * st[4]; d0b[5] -= R(2) * st[5];
-            }
-        }
-        if (strbar.c[0]) {
-            // cell strain of the LLG: e_aa = (gm + gp)(a, a) / 2, shears / 4
-            const R e0_ = strbar.c[0][c], e1 = strbar.c[1][c], e2 = strbar.c[2][c];
-            const R e3 = strbar.c[3][c], e4 = strbar.c[4][c], e5 = strbar.c[5][c];
-            T[0][0] += R(0.5) * e0_; T[1][1] += R(0.5) * e1; T[2][2] += R(0.5) * e2;
-            T[2][1] += R(0.25) * e3; T[1][2] += R(0.25) * e3;
-            T[2][0] += R(0.25) * e4; T[0][2] += R(0.25) * e4;
-            T[1][0] += R(0.25) * e5; T[0][1] += R(0.25) * e5;
-        }
-        if (back) {
-            const R mx = m.c[0][c], my = m.c[1][c], mz = m.c[2][c];
-            const R l1 = mt.l100_15, l2 = mt.l111_15;
-            ybar_m.c[0][c] += R(2) * l1 * mx * d0b[0] + l2 * (mz * d0b[4] + my * d0b[5]);
-            ybar_m.c[1][c] += R(2) * l1 * my * d0b[1] + l2 * (mz * d0b[3] + mx * d0b[5]);
-            ybar_m.c[2][c] += R(2) * l1 * mz * d0b[2] + l2 * (my * d0b[3] + mx * d0b[4]);
-        }
-    }
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-        const R l = lam_m.c[a][c];
-        adj_comb1<R>(s, l, s == 3 ? l : lamacc_m.c[a][c], ybar_m.c[a][c], lamacc_m.c[a], u_m.c[a], c);
-    }
-#pragma unroll
-    for (int d = 0; d < 3; d++)
-#pragma unroll
-        for (int a = 0; a < 3; a++) to[(d * 3 + a) * n + c] = T[d][a];
-#pragma unroll
-    for (int f = 0; f < 6; f++)
-#pragma unroll
-        for (int a = 0; a < 3; a++) to[(9 + f * 3 + a) * n + c] = O[f][a];
-}
-
-// Pass 2, per cell c: cotangent of the gradient on each of its faces that is
-// not stress-free (T of the two cells plus O of each side), then
-// ubar_a(c) = sum_d (gbar_d(lower face) - gbar_d(upper face)) / h_d
-// (g = (u(upper cell) - u(lower cell)) / h).  Written to ybar_u.
-// ybar_u is final here: the u group's RK combination (adj_comb1 at stage s)
-// follows in the same thread instead of a store of ybar_u.
+struct AdjElArgs {
+    F3T<R> fbar;
+    C6T<R> strbar;
+    F3T<R> m, ybar_m, lam_u, lamacc_u, u_u;
+    int back, s;
+};
 template <class R>
-__global__ void __launch_bounds__(256) k_adj_el_p2(Params P, const uint8_t* __restrict__ mid, const R* __restrict__ to,
-                                                  int s, F3T<R> lam_u, F3T<R> lamacc_u, F3T<R> u_u) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= P.n) return;
-    const long n = P.n;
-    R ub[3] = {R(0), R(0), R(0)};
-    const uint8_t id = mid[c];
-    if (id != 0) {
-        const int nyz = P.ny * P.nz;
-        const int i = c / nyz, j = (c - i * nyz) / P.nz, k = c - i * nyz - j * P.nz;
-        const int pos[3] = {i, j, k}, nn[3] = {P.nx, P.ny, P.nz}, per[3] = {P.per_x, P.per_y, P.per_z};
-        const int stride[3] = {nyz, P.nz, 1};
-        const R rh[3] = {R(P.rdx), R(P.rdy), R(P.rdz)};
-        for (int d = 0; d < 3; d++) {
-            const int qa = pos[d] == 0 ? nn[d] - 1 : pos[d] - 1, qb = pos[d] == nn[d] - 1 ? 0 : pos[d] + 1;
-            const int a_ = c + (qa - pos[d]) * stride[d], b_ = c + (qb - pos[d]) * stride[d];
-            const bool free_lo = (pos[d] == 0 && !per[d]) || mid[a_] == 0;
-            const bool free_hi = (pos[d] == nn[d] - 1 && !per[d]) || mid[b_] == 0;
+struct ColAdjoint {
+    const AdjElArgs<R>& A;
+    F3T<R> u;
+    R cur[6], nxt[6], yb[3], mm[3], l[3], la[3];
+    bool str;
+    __device__ __forceinline__ explicit ColAdjoint(const AdjElArgs<R>& a) : A(a), u(a.fbar), str(a.strbar.c[0] != nullptr) {
 #pragma unroll
-            for (int comp = 0; comp < 3; comp++) {
-                const int tq = (d * 3 + comp);
-                R gl = R(0), gu = R(0);
-                if (!free_lo) gl = to[tq * n + a_] + to[tq * n + c] + to[(9 + (2 * d + 1) * 3 + comp) * n + a_]
-                                   + to[(9 + (2 * d) * 3 + comp) * n + c];
-                if (!free_hi) gu = to[tq * n + c] + to[tq * n + b_] + to[(9 + (2 * d + 1) * 3 + comp) * n + c]
-                                   + to[(9 + (2 * d) * 3 + comp) * n + b_];
-                ub[comp] += (gl - gu) * rh[d];
+        for (int q = 0; q < 6; q++) cur[q] = nxt[q] = R(0);
+#pragma unroll
+        for (int a_ = 0; a_ < 3; a_++) yb[a_] = mm[a_] = l[a_] = la[a_] = R(0);
+    }
+    __device__ __forceinline__ void fetch(int c) {
+        if (!str) return;
+#pragma unroll
+        for (int q = 0; q < 6; q++) nxt[q] = A.strbar.c[q][c];
+    }
+    __device__ __forceinline__ void next() {
+#pragma unroll
+        for (int q = 0; q < 6; q++) cur[q] = nxt[q];
+    }
+    __device__ __forceinline__ void early(int c, int cl) {
+        if (c >= 0 && A.back) {
+#pragma unroll
+            for (int a = 0; a < 3; a++) { yb[a] = A.ybar_m.c[a][c]; mm[a] = A.m.c[a][c]; }
+        }
+        if (cl >= 0) {
+#pragma unroll
+            for (int a = 0; a < 3; a++) {
+                l[a] = A.lam_u.c[a][cl];
+                la[a] = A.s == 3 ? l[a] : A.lamacc_u.c[a][cl];
             }
         }
     }
+    __device__ __forceinline__ void own_terms(int, bool, const ColMat<R>&, R EN[3], R ES[3]) const {
 #pragma unroll
-    for (int a = 0; a < 3; a++) {
-        const R l = lam_u.c[a][c];
-        adj_comb1<R>(s, l, s == 3 ? l : lamacc_u.c[a][c], ub[a], lamacc_u.c[a], u_u.c[a], c);
+        for (int q = 0; q < 3; q++) { EN[q] = cur[q]; ES[q] = R(0.5) * cur[3 + q]; }
     }
+    __device__ __forceinline__ void cell(int c, bool solid, const ColMat<R>& cm, const R Tx[3], const R Ty[3], const R Tz[3]) const {
+        if (!A.back || !solid) return;
+        const R mx = mm[0], my = mm[1], mz = mm[2];
+        const R l1 = R(2) * cm.l100_15, l2 = cm.l111_15, h11 = R(0.5) * cm.c11, h12 = R(0.5) * cm.c12;
+        const R e0 = h11 * Tx[0] + h12 * (Ty[1] + Tz[2]);
+        const R e1 = h11 * Ty[1] + h12 * (Tx[0] + Tz[2]);
+        const R e2 = h11 * Tz[2] + h12 * (Tx[0] + Ty[1]);
+        const R e3 = cm.c44 * (Ty[2] + Tz[1]), e4 = cm.c44 * (Tx[2] + Tz[0]), e5 = cm.c44 * (Tx[1] + Ty[0]);
+        A.ybar_m.c[0][c] = yb[0] + (l1 * mx * e0 + l2 * (mz * e4 + my * e5));
+        A.ybar_m.c[1][c] = yb[1] + (l1 * my * e1 + l2 * (mz * e3 + mx * e5));
+        A.ybar_m.c[2][c] = yb[2] + (l1 * mz * e2 + l2 * (my * e3 + mx * e4));
+    }
+    __device__ __forceinline__ void done(int c, bool solid, const R f[3]) const {
+#pragma unroll
+        for (int a = 0; a < 3; a++) adj_comb1<R>(A.s, l[a], la[a], solid ? f[a] : R(0), A.lamacc_u.c[a], A.u_u.c[a], c);
+    }
+};
+template <class R, bool UNI>
+__global__ void __launch_bounds__(kColMaxThreads<R>, kColMinBlocks<R>)
+    k_adj_el_T(const __grid_constant__ Params P, const uint8_t* __restrict__ mid, const DevMatT<R>* __restrict__ mats,
+               const __grid_constant__ ColGeom G, int nmat, const __grid_constant__ ColMat<R> um, const __grid_constant__ AdjElArgs<R> A) {
+    GF_EXTERN_SMEM(unsigned char, smem_raw);
+    ColAdjoint<R> op(A);
+    col_march<R, UNI, kColMaxThreads<R>>(P, G, mid, mats, nmat, um, op, blockIdx.x, blockIdx.y, blockIdx.z, smem_raw);
 }
 
 // Liao extrapolation after the step (forward): the history slot of this
@@ -542,54 +493,46 @@ __global__ void k_adj_liao_pend(Params P, F3T<R> lam, R* __restrict__ pend, unsi
 
 // ybar += transposed exchange of Hbar: sum_f w_cf (ex_f Hbar_f - ex_c Hbar_c);
 // and ybar += Ms R where R is the demag convolution of Hbar (3 x n, the
-// inverse-transform output), for ferromagnetic cells.  With comb != 0 (no
-// elastodynamics) ybar is final here and the m group's RK combination
-// (adj_comb1 at stage s) follows for every cell instead of a store of ybar.
+// inverse-transform output), for ferromagnetic cells.  ybar is final here:
+// the m group's RK combination (adj_comb1 at stage s) follows for every cell
+// instead of a store of ybar.
 template <class R>
-__device__ __forceinline__ void adj_field_T_cell(const Params& P, const uint8_t* __restrict__ mid,
-                                                 const AdjMatT<R>* __restrict__ am, const R* __restrict__ aij, int nmat,
-                                                 F3T<R> hbar, const R* __restrict__ Rk, int c, V3<R>& yb) {
-    const uint8_t id = mid[c];
-    const int nyz = P.ny * P.nz;
-    const int i = c / nyz, j = (c - i * nyz) / P.nz, k = c - i * nyz - j * P.nz;
-    AdjNbr<R> n;
-    adj_neighbours(P, mid, am, aij, nmat, i, j, k, id, n);
-    const R ec = am[id - 1].ex_coef, Ms = am[id - 1].Ms;
-    const V3<R> hc = ld3(hbar, c);
-    V3<R> s = mk3<R>(R(0), R(0), R(0));
-#pragma unroll
-    for (int f = 0; f < 6; f++) {
-        if (n.w[f] == R(0)) continue;
-        const R ef = am[mid[n.nb[f]] - 1].ex_coef;
-        const V3<R> hf = ld3(hbar, n.nb[f]);
-        s.x += n.w[f] * (ef * hf.x - ec * hc.x);
-        s.y += n.w[f] * (ef * hf.y - ec * hc.y);
-        s.z += n.w[f] * (ef * hf.z - ec * hc.z);
-    }
-    yb.x += s.x; yb.y += s.y; yb.z += s.z;
-    if (Rk) { yb.x += Ms * Rk[c]; yb.y += Ms * Rk[P.n + c]; yb.z += Ms * Rk[2 * P.n + c]; }
-}
-template <class R>
-__global__ void __launch_bounds__(256) k_adj_field_T(Params P, const uint8_t* __restrict__ mid, const AdjMatT<R>* __restrict__ am,
+__global__ void __launch_bounds__(256, is_mixed<R>::value ? 4 : 3) k_adj_field_T(Params P, const uint8_t* __restrict__ mid, const AdjMatT<R>* __restrict__ am,
                                                      const R* __restrict__ aij, int nmat, F3T<R> hbar, const R* __restrict__ Rk,
-                                                     F3T<R> ybar, int comb, int s, F3T<R> lam, F3T<R> lamacc, F3T<R> u) {
+                                                     F3T<R> ybar, int s, F3T<R> lam, F3T<R> lamacc, F3T<R> u) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= P.n) return;
+    const int nyz = P.ny * P.nz;
+    const int i = c / nyz, j = (c - i * nyz) / P.nz, k = c - i * nyz - j * P.nz;
+    // loads first, as in k_adj_eval
     const uint8_t id = mid[c];
-    const bool fm = id != 0 && am[id - 1].fm;
-    if (!fm && !comb) return;
-    V3<R> yb = ld3(ybar, c);
-    if (fm) adj_field_T_cell<R>(P, mid, am, aij, nmat, hbar, Rk, c, yb);
-    if (!comb) {
-        st3(ybar, c, yb);
-        return;
-    }
-    const R ybv[3] = {yb.x, yb.y, yb.z};
+    AdjNbr<R> n;
+    adj_cells(P, i, j, k, n);
+    const V3<R> hc = ld3(hbar, c);
+    V3<R> hn[6];
 #pragma unroll
-    for (int a = 0; a < 3; a++) {
-        const R l = lam.c[a][c];
-        adj_comb1<R>(s, l, s == 3 ? l : lamacc.c[a][c], ybv[a], lamacc.c[a], u.c[a], c);
+    for (int f = 0; f < 6; f++) hn[f] = ld3(hbar, n.nb[f]);
+    V3<R> yb = ld3(ybar, c), d = mk3<R>(R(0), R(0), R(0));
+    if (Rk) d = mk3<R>(Rk[c], Rk[P.n + c], Rk[2 * P.n + c]);
+    const V3<R> lv = ld3(lam, c);
+    const V3<R> la = s == 3 ? lv : ld3(lamacc, c);
+    if (id != 0 && am[id - 1].fm) {
+        adj_weights(P, mid, am, aij, nmat, i, j, k, id, n);
+        const R ec = am[id - 1].ex_coef, Ms = am[id - 1].Ms;
+        V3<R> q = mk3<R>(R(0), R(0), R(0));
+#pragma unroll
+        for (int f = 0; f < 6; f++) {
+            if (n.w[f] == R(0)) continue;
+            const R ef = am[mid[n.nb[f]] - 1].ex_coef;
+            q.x += n.w[f] * (ef * hn[f].x - ec * hc.x);
+            q.y += n.w[f] * (ef * hn[f].y - ec * hc.y);
+            q.z += n.w[f] * (ef * hn[f].z - ec * hc.z);
+        }
+        yb.x += q.x + Ms * d.x; yb.y += q.y + Ms * d.y; yb.z += q.z + Ms * d.z;
     }
+    const R ybv[3] = {yb.x, yb.y, yb.z}, lvv[3] = {lv.x, lv.y, lv.z}, lav[3] = {la.x, la.y, la.z};
+#pragma unroll
+    for (int a = 0; a < 3; a++) adj_comb1<R>(s, lvv[a], lav[a], ybv[a], lamacc.c[a], u.c[a], c);
 }
 
 // Hbar (3 x n arrays) into the contiguous FFT input

@@ -4270,15 +4270,14 @@ struct gf_adjoint {
     double* abar = nullptr; double* hacc = nullptr; double* wbar = nullptr;   // FP64: alpha gradient, per-cell Hbar_x sum, waveform gradient
     // elastodynamics: stage u, v (stages 2-4), RK accumulators, the stage
     // force, the stage strain (LLG field), the cotangents of the force, the
-    // stage-1 force of this step (f0bar) and of fs (phi), the transposed
-    // stencil's pass-1 output (27 n), Liao history and pending cotangents
+    // stage-1 force of this step (f0bar) and of fs (phi), Liao history and
+    // pending cotangents
     double* US[3][3] = {}; double* VS[3][3] = {};
     double* UACC[3] = {}; double* VACC[3] = {};
     double* FORCE[3] = {};
     double* STR[4][6] = {};
     double* STRBAR[6] = {};
     double* FBAR[3] = {}; double* F0BAR[3] = {}; double* PHI[3] = {}; double* PHINEW[3] = {};
-    double* TO = nullptr;
     double* hist = nullptr;          // 4 slots x 12 planes (k_elastic_bc's layout)
     double* last = nullptr;          // 3 planes
     double* pend = nullptr;          // 4 slots x 3 components x 4 planes
@@ -4625,7 +4624,7 @@ int adj_step_backward(gf_adjoint* a, double* const* x, uint64_t step, bool recom
     }
     // the stage-4 cotangent u4 = lambda / 6 is read from lambda (scaled in
     // the kernels), and each group's RK combination runs in the kernel that
-    // forms the group's final ybar (vjp + field_T [+ el_p1] for m, el_p2
+    // forms the group's final ybar (vjp [+ el_T] + field_T for m, el_T
     // for u, el_vjp for v), which writes lamacc (from lambda at stage 4)
     // and the next stage's u
     for (int s = 3; s >= 0; s--) {
@@ -4638,26 +4637,32 @@ int adj_step_backward(gf_adjoint* a, double* const* x, uint64_t step, bool recom
         GF_CU(launch(k_adj_vjp<R>, dim3(bn), dim3(kThreads), 0, st, P, (const uint8_t*)eng->mid, (const AdjMatT<R>*)a->am, y,
                      v3<R>(a->HS[s]), um, us, (const R*)rp<R>(a->alpha), v3<R>(a->YBAR), v3<R>(a->HBAR), a->abar,
                      a->hacc, str, strbar));
-        const R* Rk = nullptr;
-        if (eng->demag_mode == 0) GF_TRY(adj_demag_T<R>(a, Rk));
-        GF_CU(launch(k_adj_field_T<R>, dim3(bn), dim3(kThreads), 0, st, P, (const uint8_t*)eng->mid, (const AdjMatT<R>*)a->am,
-                     (const R*)rp<R>(a->aij), a->nmat, v3<R>(a->HBAR), Rk, v3<R>(a->YBAR), a->el ? 0 : 1, s, v3<R>(a->LAM),
-                     v3<R>(a->LAMACC), v3<R>(a->U)));
         if (a->el) {
             // elastic increments (and the v group's combination), then the
-            // transposed stress and strain stencils (the m and u groups')
+            // transposed stress and strain stencils (the u group's)
             cudaError_t e;
             if (s == 3) e = adj_el_vjp_launch<3, R>(a);
             else if (s == 2) e = adj_el_vjp_launch<2, R>(a);
             else if (s == 1) e = adj_el_vjp_launch<1, R>(a);
             else e = adj_el_vjp_launch<0, R>(a);
             GF_CU(e);
-            GF_CU(launch(k_adj_el_p1<R>, dim3(bn), dim3(kThreads), 0, st, P, (const uint8_t*)eng->mid, adj_mats<R>(eng),
-                         v3<R>(a->FBAR), strbar, y, v3<R>(a->YBAR), (int)P.elasto_back, rp<R>(a->TO), s, v3<R>(a->LAM),
-                         v3<R>(a->LAMACC), v3<R>(a->U)));
-            GF_CU(launch(k_adj_el_p2<R>, dim3(bn), dim3(kThreads), 0, st, P, (const uint8_t*)eng->mid, (const R*)rp<R>(a->TO),
-                         s, v3<R>(a->LAM + 3), v3<R>(a->LAMACC + 3), v3<R>(a->U + 3)));
+            AdjElArgs<R> A;
+            A.fbar = v3<R>(a->FBAR); A.strbar = strbar; A.m = y; A.ybar_m = v3<R>(a->YBAR);
+            A.lam_u = v3<R>(a->LAM + 3); A.lamacc_u = v3<R>(a->LAMACC + 3); A.u_u = v3<R>(a->U + 3);
+            A.back = (int)P.elasto_back; A.s = s;
+            const ColGeom& g = eng->el_geom;
+            const size_t sm = col_smem_bytes<R>(kColMaxThreads<R>, eng->el_nmat);
+            auto el_T = [&](auto k) {
+                return launch_tiled(k, col_grid(eng), dim3(g.threads), sm, st, P, (const uint8_t*)eng->mid, adj_mats<R>(eng), g,
+                                    eng->el_nmat, col_um<R>(eng), A);
+            };
+            GF_CU(eng->uni ? el_T(k_adj_el_T<R, true>) : el_T(k_adj_el_T<R, false>));
         }
+        const R* Rk = nullptr;
+        if (eng->demag_mode == 0) GF_TRY(adj_demag_T<R>(a, Rk));
+        GF_CU(launch(k_adj_field_T<R>, dim3(bn), dim3(kThreads), 0, st, P, (const uint8_t*)eng->mid, (const AdjMatT<R>*)a->am,
+                     (const R*)rp<R>(a->aij), a->nmat, v3<R>(a->HBAR), Rk, v3<R>(a->YBAR), s, v3<R>(a->LAM),
+                     v3<R>(a->LAMACC), v3<R>(a->U)));
     }
     for (int c = 0; c < 3 * ng; c++) std::swap(a->LAM[c], a->LAMACC[c]);
     if (a->el) {
@@ -4871,6 +4876,7 @@ int gf_adjoint_create(gf_engine* e, int n_wave, int checkpoint_every, gf_adjoint
         if (d.abc_1D) { eng->err = "the adjoint covers the Liao boundary of the elastic run, not the Mur one (if_1D_ABC)"; return GF_EUNSUPPORTED; }
         if (d.strain_pulse) { eng->err = "the adjoint does not cover the elastic strain source"; return GF_EUNSUPPORTED; }
         if (P.ny < P.nz) { eng->err = "the adjoint needs ny >= nz (the reference's z-face neighbour rule for k = ny-1 is not transposed)"; return GF_EUNSUPPORTED; }
+        if (!eng->el_col) { eng->err = "the adjoint needs cubic materials in the unrotated frame"; return GF_EUNSUPPORTED; }
         if (P.nz < 5) { eng->err = "the adjoint's Liao boundary needs nz >= 5"; return GF_EUNSUPPORTED; }
         if (eng->es_eps[0] || eng->es_eig[0]) { eng->err = "the adjoint does not cover static strain inputs"; return GF_EUNSUPPORTED; }
     }
@@ -4936,7 +4942,14 @@ int gf_adjoint_create(gf_engine* e, int n_wave, int checkpoint_every, gf_adjoint
                 if ((rc = adj_alloc(a, &a->STR[s_][q], (size_t)n)) != GF_OK) return fail(rc);
         for (int q = 0; q < 6; q++)
             if ((rc = adj_alloc(a, &a->STRBAR[q], (size_t)n)) != GF_OK) return fail(rc);
-        if ((rc = adj_alloc(a, &a->TO, (size_t)27 * n)) != GF_OK) return fail(rc);
+        // the adjoint's decks are unrotated with ny >= nz: col_path holds
+        cudaError_t ce = cudaSuccess;
+        auto opt_in = [&](auto k, size_t sm) {
+            if (ce == cudaSuccess) ce = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        };
+        if (a->f32) { opt_in(k_adj_el_T<float, true>, col_smem_bytes<float>(kColMaxThreads<float>, kMaxMat)); opt_in(k_adj_el_T<float, false>, col_smem_bytes<float>(kColMaxThreads<float>, kMaxMat)); }
+        else { opt_in(k_adj_el_T<double, true>, col_smem_bytes<double>(kColMaxThreads<double>, kMaxMat)); opt_in(k_adj_el_T<double, false>, col_smem_bytes<double>(kColMaxThreads<double>, kMaxMat)); }
+        if (ce != cudaSuccess) { eng->err = std::string("adjoint: ") + cudaGetErrorString(ce); return fail(GF_ECUDA); }
         if ((rc = adj_alloc(a, &a->hist, (size_t)48 * plane)) != GF_OK) return fail(rc);
         if ((rc = adj_alloc(a, &a->last, (size_t)3 * plane)) != GF_OK) return fail(rc);
         if ((rc = adj_alloc(a, &a->pend, (size_t)48 * plane)) != GF_OK) return fail(rc);

@@ -183,3 +183,31 @@ def test_yee_update_equals_the_general_one(gf, name, precision):
     pole = dataclasses.replace(D.ggg(), drude=((1.0, 1e15, 1e-14), (0.0, 0.0, 1.0), (0.0, 0.0, 1.0)))
     g = dataclasses.replace(d, materials=list(d.materials) + [pole])
     _same(_run(gf, d, precision), _run(gf, g, precision), TOL[precision])
+
+
+def test_adjoint_of_a_layered_film_matches_finite_differences(gf, tmp_path):
+    """The transposed elastic march with several materials and vacuum."""
+    from test_gpu_adjoint import MU0, _grads
+    steps, nw = 60, 4
+    D = gf.decks
+    d = D.preset_fm_demag(nx=6, ny=12, nz=11, steps=steps)
+    d.Hext_table = None
+    d.Hext_stat = (0.0, 0.0, 1.0 / MU0)
+    film = D.yig(0.02, magnetoelastic=True)
+    film.lam100 *= 1000.0
+    film.lam111 *= 1000.0
+    d.materials = [film, dataclasses.replace(D.ggg(), c44=1.3e11, stiff_damping=2e-13, mass_damping=1e9)]
+    d.layers = [(4, 2), (5, 1), (2, 0)]
+    mc = d.material_cell()
+    d.m0 = D.tilt_m0((6, 12, 11), 31, mc == 1, 10.0)
+    d.elastic, d.elasto_back, d.elasto_on = True, True, True
+    D.write_deck(d, str(tmp_path))
+    alpha0 = 0.02 * (1.0 + 0.1 * np.random.default_rng(5).random(d.n)) * (mc.ravel() == 1)
+    tt = (np.arange(nw) + 0.5) / nw
+    wave0 = (1e-2 / MU0) * np.sin(2 * np.pi * tt)
+    gw, ga, (fd_w, v, fd_a) = _grads(gf, tmp_path, d, steps, nw, wave0, alpha0, True)
+    assert np.max(np.abs(gw - fd_w)) <= 1e-4 * np.max(np.abs(fd_w))
+    assert abs(float(ga @ v) - fd_a) <= 1e-4 * abs(fd_a)
+    gw32, ga32, _ = _grads(gf, tmp_path, d, steps, nw, wave0, alpha0, False, precision="mixed")
+    assert np.max(np.abs(gw32 - gw)) <= 1e-3 * np.max(np.abs(gw))
+    assert np.max(np.abs(ga32 - ga)) <= 1e-3 * np.max(np.abs(ga))
