@@ -38,6 +38,7 @@
 #include "gf_fe.cuh"
 #include "gf_em.cuh"
 #include "gf_demag.cuh"
+#include "gf_conv.cuh"
 #include "gf_util.cuh"
 #include "gf_adjoint.cuh"
 #include "gf_batch.cuh"
@@ -134,6 +135,11 @@ struct gf_engine {
     // k_elastic_col runs the stress divergence (col_path), and its tile
     bool el_col = false;
     ColGeom el_geom = {};
+    // the per-stage magnetostatic convolution by the engine's own transforms
+    // (gf_conv.cuh): geometry and twiddles
+    bool conv = false;
+    ConvGeom cg = {};
+    void* conv_tw = nullptr;
     double* liao_hist = nullptr; double* liao_last = nullptr;
     double* scratch = nullptr;             // output staging (scratch_main doubles), then reduction partials
     size_t scratch_main = 0;
@@ -209,6 +215,7 @@ struct gf_engine {
 int gf_mixed_enqueue_step(gf_engine* eng, int parity);                 // kernels of one step, mixed form
 int gf_mixed_enqueue_stage(gf_engine* eng, int parity, int s);         // kernels of stage s (0..3), mixed form
 int gf_mixed_elastic_setup(gf_engine* eng, int smem, int* per_sm);   // shared-memory opt-in, occupancy
+int gf_mixed_conv_attr(gf_engine* eng);                                 // shared-memory opt-in of the convolution kernels
 int gf_mixed_col_setup(gf_engine* eng);                                 // the same for k_elastic_col, and its tile
 int gf_mixed_time_tile(gf_engine* eng, int reps, float* ms);          // stage-1 elastic tile, mean ms per launch
 int gf_mixed_adj_elastic(gf_engine* eng, int s, int rk, const StageIOT<float>& io);  // adjoint: FP32 elastic tile / RK of stage s
@@ -993,6 +1000,36 @@ template <> const StageIOT<double>& stage_io<double>(const gf_engine* eng, int p
 template <> const LLGTablesT<double>* llg_tables<double>(const gf_engine* eng) { return eng->llg_tab; }
 #endif
 
+// shared-memory opt-in of the convolution kernels (of this translation unit)
+template <class R>
+int conv_attr(gf_engine* eng) {
+    GF_CU(cudaFuncSetAttribute(k_conv_fwd<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kConvMaxSmem));
+    GF_CU(cudaFuncSetAttribute(k_conv_x<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kConvMaxSmem));
+    GF_CU(cudaFuncSetAttribute(k_conv_inv<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kConvMaxSmem));
+    return GF_OK;
+}
+
+// out = the demag convolution of Ms in (scale: in is m, FM cells) or of in
+template <class R>
+int conv_solve(gf_engine* eng, F3T<R> in, bool scale, F3T<R> out, bool counted) {
+    const ConvGeom& g = eng->cg;
+    cudaStream_t st = eng->stream;
+    auto L = [&](const char* name, auto k, dim3 gr, int th, size_t sm, auto... args) -> cudaError_t {
+        return counted ? klaunch(eng, name, k, gr, dim3((unsigned)th), sm, st, args...) : launch(k, gr, dim3((unsigned)th), sm, st, args...);
+    };
+    const DevMatT<R>* mats = nullptr;
+    const ConvTensor<R>* N;
+    if constexpr (is_mixed<R>::value) { if (scale) mats = eng->mats_f; N = eng->Nr; }
+    else { if (scale) mats = eng->mats; N = eng->Nk; }
+    const Cx<R>* tw = static_cast<const Cx<R>*>(eng->conv_tw);
+    Cx<R>* spec = reinterpret_cast<Cx<R>*>(eng->Mk);
+    const dim3 planes((unsigned)g.nx, 3u);
+    GF_CU(L("k_conv_fwd", k_conv_fwd<R>, planes, kConvThreads, conv_plane_smem<R>(g), g, in, (const uint8_t*)eng->mid, mats, (int)eng->deck.mats.size(), tw, spec));
+    GF_CU(L("k_conv_x", k_conv_x<R>, dim3((unsigned)g.groups), kConvThreads, conv_x_smem<R>(g), g, tw, N, (R)(-1. / (eng->P.dx * eng->P.dy * eng->P.dz)), spec));
+    GF_CU(L("k_conv_inv", k_conv_inv<R>, planes, kConvThreads, conv_plane_smem<R>(g), g, tw, (const Cx<R>*)spec, out));
+    return GF_OK;
+}
+
 // magnetostatic field of magnetisation m into Hstat (FFT, demag factors or
 // the 1-D model), FP64 form
 // src_ready: the stage's LLG kernel has already written the transform's
@@ -1004,10 +1041,13 @@ int demag_solve(gf_engine* eng, F3 m, F3 a1, F3 a2, bool counted, bool src_ready
     auto L = [&](const char* name, auto k, dim3 g, dim3 b, auto... args) -> cudaError_t {
         return counted ? klaunch(eng, name, k, g, b, 0, st, args...) : launch(k, g, b, 0, st, args...);
     };
-    if (eng->demag_mode == 0) {
+    if (eng->demag_mode == 0 && eng->conv && !P.afm && !src_ready) {
+        GF_TRY(conv_solve<double>(eng, m, true, f3(eng->Hstat), counted));
+    } else if (eng->demag_mode == 0) {
         if (!src_ready)
             GF_CU(L("k_mag_source", k_mag_source, dim3(bn), dim3(kThreads), P, (const DevMat*)eng->mats, (const uint8_t*)eng->mid,
                     m, a1, a2, 0, eng->Mfft, f3(eng->Hstat), 0., 0., 0.));
+        if (eng->conv) return conv_solve<double>(eng, f3(eng->Hstat), false, f3(eng->Hstat), counted);
         GF_FFT(cufftExecD2Z(eng->plan_r2c, eng->Mfft, eng->Mk));
         const long n21 = (long)P.nx * P.ny * (P.nz / 2 + 1);
         const double vol_neg = -P.dx * P.dy * P.dz;
@@ -1034,10 +1074,13 @@ int demag_solve_f32(gf_engine* eng, F3T<float> m, F3T<float> a1, F3T<float> a2, 
     };
     float* M3 = reinterpret_cast<float*>(eng->Mfft);
     cufftComplex* Mk = reinterpret_cast<cufftComplex*>(eng->Mk);
-    if (eng->demag_mode == 0) {
+    if (eng->demag_mode == 0 && eng->conv && !P.afm && !src_ready) {
+        GF_TRY(conv_solve<float>(eng, m, true, f3f(eng->Hstat), counted));
+    } else if (eng->demag_mode == 0) {
         if (!src_ready)
             GF_CU(L("k_mag_source", k_mag_source_f32, dim3(bn), dim3(kThreads), P, (const DevMatT<float>*)eng->mats_f,
                     (const uint8_t*)eng->mid, m, a1, a2, 0, M3, f3f(eng->Hstat), 0.f, 0.f, 0.f));
+        if (eng->conv) return conv_solve<float>(eng, f3f(eng->Hstat), false, f3f(eng->Hstat), counted);
         GF_FFT(cufftExecR2C(eng->plan_r2c, M3, Mk));
         const long n21 = (long)P.nx * P.ny * (P.nz / 2 + 1);
         const float inv_vol_neg = (float)(-1. / (P.dx * P.dy * P.dz));
@@ -1326,6 +1369,7 @@ int gf_mixed_elastic_setup(gf_engine* eng, int smem, int* per_sm) {
     return GF_OK;
 }
 
+int gf_mixed_conv_attr(gf_engine* eng) { return conv_attr<float>(eng); }
 int gf_mixed_col_setup(gf_engine* eng) { return col_setup<float>(eng); }
 
 int gf_mixed_time_tile(gf_engine* eng, int reps, float* ms) { return time_tile_t<float>(eng, reps, ms); }
@@ -1491,6 +1535,57 @@ std::shared_ptr<const std::vector<double>> newell_tables(const Params& P) {
     return last;
 }
 
+// buffers of the convolution: M_k, H (3n, H_stat is a view of it), the
+// twiddles of the three lengths, and the tensor's spectra from the host's FP64
+// tables (a temporary cuFFT plan; FP32 keeps the six real ones)
+template <class R>
+int conv_setup(gf_engine* eng) {
+    const Params& P = eng->P;
+    const long n = P.n, nk = eng->cg.nk;
+    int dims[3] = {P.nx, P.ny, P.nz};
+    GF_TRY(dalloc(eng, reinterpret_cast<void**>(&eng->Mfft), sizeof(R) * 3 * (size_t)n));
+    GF_TRY(dalloc(eng, reinterpret_cast<void**>(&eng->Mk), sizeof(Cx<R>) * 3 * (size_t)nk));
+    if constexpr (is_mixed<R>::value) GF_TRY(dalloc(eng, reinterpret_cast<void**>(&eng->Nr), sizeof(float) * 6 * (size_t)nk));
+    else GF_TRY(dalloc_n(eng, &eng->Nk, (size_t)9 * nk));
+    for (int a = 0; a < 3; a++) eng->Hstat[a] = reinterpret_cast<double*>(reinterpret_cast<R*>(eng->Mfft) + (size_t)a * n);
+    std::vector<Cx<R>> tw;
+    for (int len : {P.nx, P.ny, P.nz})
+        for (int k = 0; k < len; k++) {
+            const double ph = -2. * kPi * (double)k / (double)len;
+            tw.push_back(Cx<R>{(R)std::cos(ph), (R)std::sin(ph)});
+        }
+    GF_TRY(dalloc(eng, &eng->conv_tw, sizeof(Cx<R>) * tw.size()));
+    GF_CU(cudaMemcpy(eng->conv_tw, tw.data(), sizeof(Cx<R>) * tw.size(), cudaMemcpyHostToDevice));
+    GF_TRY(conv_attr<R>(eng));
+    if (eng->mixed) GF_TRY(gf_mixed_conv_attr(eng));
+    const std::shared_ptr<const std::vector<double>> host_tab = newell_tables(P);
+    double* tab = nullptr;
+    cufftDoubleComplex* nk64 = nullptr;
+    cufftHandle p64 = 0;
+    cudaError_t ce = cudaMalloc(&tab, sizeof(double) * 9 * (size_t)n);
+    if constexpr (is_mixed<R>::value) { if (ce == cudaSuccess) ce = cudaMalloc(&nk64, sizeof(cufftDoubleComplex) * 9 * (size_t)nk); }
+    cufftDoubleComplex* spec = is_mixed<R>::value ? nk64 : eng->Nk;
+    cufftResult fr = CUFFT_SUCCESS;
+    if (ce == cudaSuccess) fr = cufftPlanMany(&p64, 3, dims, nullptr, 1, (int)n, nullptr, 1, (int)nk, CUFFT_D2Z, 3);
+    if (ce == cudaSuccess && fr == CUFFT_SUCCESS) fr = cufftSetStream(p64, eng->stream);
+    if (ce == cudaSuccess && fr == CUFFT_SUCCESS)
+        ce = cudaMemcpyAsync(tab, host_tab->data(), sizeof(double) * 9 * (size_t)n, cudaMemcpyHostToDevice, eng->stream);
+    for (int b = 0; b < 3 && ce == cudaSuccess && fr == CUFFT_SUCCESS; b++)
+        fr = cufftExecD2Z(p64, tab + (size_t)3 * b * n, spec + (size_t)3 * b * nk);
+    if constexpr (is_mixed<R>::value) {
+        if (ce == cudaSuccess && fr == CUFFT_SUCCESS)
+            ce = launch(k_spectra_real<R>, dim3(blocks_for(nk, kThreads)), dim3(kThreads), 0, eng->stream, (const cuDoubleComplex*)nk64, nk,
+                        eng->Nr);
+    }
+    if (ce == cudaSuccess) ce = cudaStreamSynchronize(eng->stream);
+    if (p64) cufftDestroy(p64);
+    if (tab) cudaFree(tab);
+    if (nk64) cudaFree(nk64);
+    if (ce != cudaSuccess) { eng->err = std::string("demag tables: ") + cudaGetErrorString(ce); return GF_ECUDA; }
+    if (fr != CUFFT_SUCCESS) { eng->err = "demag tables: cuFFT error " + std::to_string((int)fr); return GF_ECUDA; }
+    return GF_OK;
+}
+
 int setup_demag(gf_engine* eng) {
     const Deck& d = eng->deck;
     const Params& P = eng->P;
@@ -1507,6 +1602,15 @@ int setup_demag(gf_engine* eng) {
     if (eng->demag_mode != 0) return GF_OK;
     const long n21 = (long)P.nx * P.ny * (P.nz / 2 + 1);
     int dims[3] = {P.nx, P.ny, P.nz};
+    // the engine's own transforms where a stage solves for the field; a
+    // field frozen at set-up (Maxwell runs) keeps cuFFT and, in FP64, the
+    // reference's nine spectra
+    eng->conv = eng->demag_per_stage &&
+                (eng->mixed ? conv_geom<float>(P.nx, P.ny, P.nz, eng->cg) && conv_pays<float>(eng->cg, d.elastodynamics)
+                            : conv_geom<double>(P.nx, P.ny, P.nz, eng->cg) && conv_pays<double>(eng->cg, d.elastodynamics));
+    if (eng->conv) {
+        return eng->mixed ? conv_setup<float>(eng) : conv_setup<double>(eng);
+    }
     if (eng->mixed) {
         // M (3n real), M_k (3 n21 complex) and the six real spectra in FP32
         GF_TRY(dalloc(eng, reinterpret_cast<void**>(&eng->Mfft), sizeof(float) * 3 * (size_t)P.n));
@@ -4351,6 +4455,10 @@ int adj_demag(gf_adjoint* a, F3T<R> y, F3T<R>& hd) {
     gf_engine* eng = a->eng;
     const Params& P = eng->P;
     if (eng->demag_mode != 0) { hd = v3c<R>(rp<R>(a->zero3), P.n); return GF_OK; }
+    if (eng->conv) {
+        hd = v3c<R>(rp<R>(eng->Mfft), P.n);
+        return conv_solve<R>(eng, y, true, hd, false);
+    }
     cudaStream_t st = eng->stream;
     const long n21 = (long)P.nx * P.ny * (P.nz / 2 + 1);
     if constexpr (is_mixed<R>::value) {
@@ -4386,6 +4494,10 @@ int adj_demag_T(gf_adjoint* a, const R*& out) {
     const unsigned bn = blocks_for(P.n, kThreads);
     const long n21 = (long)P.nx * P.ny * (P.nz / 2 + 1);
     R* M3 = reinterpret_cast<R*>(eng->Mfft);
+    if (eng->conv) {
+        out = M3;
+        return conv_solve<R>(eng, v3<R>(a->HBAR), false, v3c<R>(M3, P.n), false);
+    }
     GF_CU(launch(k_adj_pack<R>, dim3(bn), dim3(kThreads), 0, st, P, v3<R>(a->HBAR), M3));
     if constexpr (is_mixed<R>::value) {
         cufftComplex* Mk = reinterpret_cast<cufftComplex*>(eng->Mk);

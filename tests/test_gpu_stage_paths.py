@@ -185,6 +185,45 @@ def test_yee_update_equals_the_general_one(gf, name, precision):
     _same(_run(gf, d, precision), _run(gf, g, precision), TOL[precision])
 
 
+# sides with the transforms' radices 8, 4, 2, 3, 5 and their products, odd
+# ones, a single plane, row or layer, and (49, 22, 250) three that cuFFT keeps
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("shape", [(8, 6, 4), (5, 3, 2), (64, 16, 8), (30, 18, 10), (24, 45, 9), (128, 5, 3), (4, 4, 1), (1, 16, 6),
+                                   (20, 1, 5), (90, 2, 15), (49, 6, 4), (6, 22, 4), (250, 3, 2)])
+def test_stage_convolution_matches_the_restatement(gf, shape, precision):
+    from oracle import restate_fm
+    nx, ny, nz = shape
+    d = gf.decks.preset_fm_demag(nx=nx, ny=ny, nz=nz, steps=10)
+    d.m0 = _unit(np.random.default_rng(23), shape)
+    with gf.Engine.from_params(d, device=0, precision=precision) as e:
+        got = [e.download("Hstat")]
+        e.advance(1)
+        got.append(e.download("Hstat"))
+        m1 = e.download("m")
+    Nk = restate_fm.demag_spectra(nx, ny, nz, d.dx, d.dy, d.dz)
+    for H, m in zip(got, (d.m0, m1)):
+        ref = restate_fm.h_static(Nk, d.materials[0].Ms * m, d.dx, d.dy, d.dz)
+        # FP64: rounding of the tables' far field (small differences of large
+        # terms) between two libms; FP32: log2(n) roundings of 6e-8
+        assert np.linalg.norm(H - ref) <= {"fp64": 1e-9, "mixed": 3e-6}[precision] * np.linalg.norm(ref)
+
+
+def test_stage_convolution_covers_only_magnetic_cells(gf):
+    """A film over a non-magnetic substrate: the source is Ms m in the film."""
+    from oracle import restate_fm
+    d = gf.decks.preset_fm_demag(nx=12, ny=10, nz=8, steps=10)
+    d.materials = [gf.decks.ggg(), gf.decks.yig(1e-2)]
+    d.layers = [(3, 1), (4, 2), (1, 0)]
+    mag = d.material_cell() == 2
+    d.m0 = _unit(np.random.default_rng(29), (12, 10, 8)) * mag
+    Nk = restate_fm.demag_spectra(12, 10, 8, d.dx, d.dy, d.dz)
+    ref = restate_fm.h_static(Nk, d.materials[1].Ms * d.m0, d.dx, d.dy, d.dz)
+    for precision, tol in (("fp64", 1e-9), ("mixed", 3e-6)):
+        with gf.Engine.from_params(d, device=0, precision=precision) as e:
+            H = e.download("Hstat")
+        assert np.linalg.norm(H - ref) <= tol * np.linalg.norm(ref)
+
+
 def test_adjoint_of_a_layered_film_matches_finite_differences(gf, tmp_path):
     """The transposed elastic march with several materials and vacuum."""
     from test_gpu_adjoint import MU0, _grads
