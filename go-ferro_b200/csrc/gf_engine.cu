@@ -1609,6 +1609,8 @@ int setup_demag(gf_engine* eng) {
                 (eng->mixed ? conv_geom<float>(P.nx, P.ny, P.nz, eng->cg) && conv_pays<float>(eng->cg, d.elastodynamics)
                             : conv_geom<double>(P.nx, P.ny, P.nz, eng->cg) && conv_pays<double>(eng->cg, d.elastodynamics));
     if (eng->conv) {
+        // k_conv_fwd forms Ms m itself: the LLG kernel writes m only
+        eng->demag_src_fused = false;
         return eng->mixed ? conv_setup<float>(eng) : conv_setup<double>(eng);
     }
     if (eng->mixed) {

@@ -60,17 +60,65 @@ struct LLGMat {
 #define GF_LLG_MINB_F32 4
 #endif
 #ifndef GF_LLG_MINB_F64
-#define GF_LLG_MINB_F64 4
+#define GF_LLG_MINB_F64 2
 #endif
 template <int S, class R = double>
-// (256, 4): 64 registers, 32 resident warps per SM for its neighbour-load
-// latency; measured faster than 98 registers at 16 warps despite a few spills
-// (with the RK operands gathered before the first store, on the 128x128x96
-// magnetoelastic film: FP64 0.225 ms per step at 4 blocks, 0.238 at 3, 0.285
-// at 2; FP32 0.145 at 4)
+// Every operand is loaded before its first use: 64 registers hold them in FP32
+// (4 blocks per SM), 126 in FP64 (2).  us per launch before (loads where they
+// were used, 64 registers in both) and now: 128x128x96 magnetoelastic film 49
+// -> 44 FP64 and 34 -> 30 FP32, 256x256x32 film FP32 86 -> 67; ms per step:
+// 120x90x20 FP64 0.165 -> 0.153, 128x128x32 FP64 0.308 -> 0.289.  FP64 with
+// only the neighbours' m ahead of the barrier: 47 at 3 blocks, 53 at 4; FP32 at
+// 3 blocks 74 on the 256x256x32 film.
 __global__ void __launch_bounds__(256, is_mixed<R>::value ? GF_LLG_MINB_F32 : GF_LLG_MINB_F64) k_llg_fm(Params P, StageIOT<R> io, const LLGTablesT<R>* __restrict__ tab, int nmat) {
     __shared__ LLGMat<R> mt[kMaxMat];
     __shared__ R sA[kMaxMat + 1][kMaxMat + 1];
+    const int bjk = (int)(P.fm_bj * P.fm_bk);
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x;
+    const int t = min(tid, bjk - 1);
+    const int bj = t / (int)P.fm_bk;
+    const int i = (int)P.fm_i0 + blockIdx.y, j = (int)P.fm_j0 + bj, k = (int)P.fm_k0 + (t - bj * (int)P.fm_bk);
+    const int nx = P.nx, ny = P.ny, nz = P.nz;
+    const int c = (i * ny + j) * nz + k;
+    const R zero = R(0);
+
+    // Every operand is loaded before the first use and before the barrier of
+    // the material tables, so that one memory latency covers them.
+    const uint8_t id = io.mid[c];
+    const R mxc = io.m_in.c[0][c], myc = io.m_in.c[1][c], mzc = io.m_in.c[2][c];
+    // neighbour ids and m with periodic wrap at array ends (the wrapped
+    // indices are always inside the array)
+    const int ib = (i == 0) ? nx - 1 : i - 1, iF = (i == nx - 1) ? 0 : i + 1;
+    const int jb = (j == 0) ? ny - 1 : j - 1, jF = (j == ny - 1) ? 0 : j + 1;
+    const int kb = (k == 0) ? nz - 1 : k - 1, kF = (k == nz - 1) ? 0 : k + 1;
+    const int cxb = (ib * ny + j) * nz + k, cxf = (iF * ny + j) * nz + k;
+    const int cyb = (i * ny + jb) * nz + k, cyf = (i * ny + jF) * nz + k;
+    const int czb = (i * ny + j) * nz + kb, czf = (i * ny + j) * nz + kF;
+    R nm[6][3];
+    {
+        const int ncell[6] = {cxb, cxf, cyb, cyf, czb, czf};
+#pragma unroll
+        for (int f = 0; f < 6; f++)
+#pragma unroll
+            for (int a = 0; a < 3; a++) nm[f][a] = io.m_in.c[a][ncell[f]];
+    }
+    const uint8_t idxb = io.mid[cxb], idxf = io.mid[cxf], idyb = io.mid[cyb], idyf = io.mid[cyf];
+    const uint8_t idzb = io.mid[czb], idzf = io.mid[czf];
+    R exx = zero, eyy = zero, ezz = zero, eyz = zero, exz = zero, exy = zero;
+    if (P.elasto_on) {
+        R e[6];
+        cell_strain_total(P, io, i, j, k, c, e);
+        exx = e[0]; eyy = e[1]; ezz = e[2]; eyz = e[3]; exz = e[4]; exy = e[5];
+    }
+    R hs[3], mx0[3], ma[3], mcm[3];
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        hs[a] = io.Hstat.c[a][c];
+        mx0[a] = io.m_x.c[a][c];
+        ma[a] = (S > 0) ? io.m_acc.c[a][c] : R(0.);
+        mcm[a] = R(0.);
+        if constexpr (is_mixed<R>::value) { if (S == 3) mcm[a] = io.m_cmp.c[a][c]; }
+    }
     for (int q = threadIdx.x; q < nmat; q += blockDim.x) {
         const DevMatT<R>& d = io.mats[q];
         mt[q] = LLGMat<R>{d.Aex, d.dA, d.ex_coef, d.dmi_coef, d.K1c, d.K2c, d.B1c, d.B2c, d.precess, d.alpha_precess, d.Ms,
@@ -81,55 +129,19 @@ __global__ void __launch_bounds__(256, is_mixed<R>::value ? GF_LLG_MINB_F32 : GF
         sA[a][b] = tab->Aij[a][b];
     }
     __syncthreads();
-    const int bjk = (int)(P.fm_bj * P.fm_bk);
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= bjk) return;
-    const int bj = t / (int)P.fm_bk;
-    const int i = (int)P.fm_i0 + blockIdx.y, j = (int)P.fm_j0 + bj, k = (int)P.fm_k0 + (t - bj * (int)P.fm_bk);
-    const int nx = P.nx, ny = P.ny, nz = P.nz;
-    const int c = (i * ny + j) * nz + k;
+    if (tid >= bjk) return;
     auto fm_at = [&](uint8_t q) { return q != 0 && mt[q - 1].fm != 0u; };
-    const R zero = R(0);
 
-    const uint8_t id = io.mid[c];
     const bool fm_cell = fm_at(id);
     R dmx = zero, dmy = zero, dmz = zero;
-    const R mxc = io.m_in.c[0][c], myc = io.m_in.c[1][c], mzc = io.m_in.c[2][c];
     if (fm_cell) {
         const LLGMat<R>& mat = mt[id - 1];
         R mx, my, mz;
         glb2crt(P, mxc, myc, mzc, mx, my, mz);
 
-        R exx = zero, eyy = zero, ezz = zero, eyz = zero, exz = zero, exy = zero;
-        if (P.elasto_on) {
-            R e[6];
-            cell_strain_total(P, io, i, j, k, c, e);
-            exx = e[0]; eyy = e[1]; ezz = e[2]; eyz = e[3]; exz = e[4]; exy = e[5];
-        }
-
         // ---- one-sided differences with interface slopes ----
         const R A = mat.Aex;
         const R dA = mat.dA;   // D/2./A
-        // neighbour ids and linear indices with periodic wrap at array ends
-        const int ib = (i == 0) ? nx - 1 : i - 1, iF = (i == nx - 1) ? 0 : i + 1;
-        const int jb = (j == 0) ? ny - 1 : j - 1, jF = (j == ny - 1) ? 0 : j + 1;
-        const int kb = (k == 0) ? nz - 1 : k - 1, kF = (k == nz - 1) ? 0 : k + 1;
-        const int cxb = (ib * ny + j) * nz + k, cxf = (iF * ny + j) * nz + k;
-        const int cyb = (i * ny + jb) * nz + k, cyf = (i * ny + jF) * nz + k;
-        const int czb = (i * ny + j) * nz + kb, czf = (i * ny + j) * nz + kF;
-        // the six neighbours' m is loaded whether or not the face is a surface
-        // (the wrapped indices are always inside the array), so these loads do
-        // not wait for the neighbour ids
-        R nm[6][3];
-        {
-            const int ncell[6] = {cxb, cxf, cyb, cyf, czb, czf};
-#pragma unroll
-            for (int f = 0; f < 6; f++)
-#pragma unroll
-                for (int a = 0; a < 3; a++) nm[f][a] = io.m_in.c[a][ncell[f]];
-        }
-        const uint8_t idxb = io.mid[cxb], idxf = io.mid[cxf], idyb = io.mid[cyb], idyf = io.mid[cyf];
-        const uint8_t idzb = io.mid[czb], idzf = io.mid[czf];
         // a face is an FM surface when the neighbour across it is not FM, or
         // it is a non-periodic system boundary
         const bool sxb = (i == 0 && !P.per_x) || !fm_at(idxb);
@@ -201,9 +213,9 @@ __global__ void __launch_bounds__(256, is_mixed<R>::value ? GF_LLG_MINB_F32 : GF
         const StageDrive& dr = stage_drive(io, S);
         R hnx = zero, hny = zero, hnz = zero;
         if (P.has_hext_nonunif) { hnx = io.Hnu.c[0][c]; hny = io.Hnu.c[1][c]; hnz = io.Hnu.c[2][c]; }
-        R Hx = io.Hstat.c[0][c] + Hax + Hmx + Hex[0] + Hdx + R(dr.Hext[0]) + hnx;
-        R Hy = io.Hstat.c[1][c] + Hay + Hmy + Hex[1] + Hdy + R(dr.Hext[1]) + hny;
-        R Hz = io.Hstat.c[2][c] + Haz + Hmz + Hex[2] + Hdz + R(dr.Hext[2]) + hnz;
+        R Hx = hs[0] + Hax + Hmx + Hex[0] + Hdx + R(dr.Hext[0]) + hnx;
+        R Hy = hs[1] + Hay + Hmy + Hex[1] + Hdy + R(dr.Hext[1]) + hny;
+        R Hz = hs[2] + Haz + Hmz + Hex[2] + Hdz + R(dr.Hext[2]) + hnz;
 
         if (P.em_back_M) {
             // cell-centred Maxwell H of the stage state (EMdynamic_solver.cpp:3780-3810)
@@ -215,7 +227,7 @@ __global__ void __launch_bounds__(256, is_mixed<R>::value ? GF_LLG_MINB_F32 : GF
             // with the 1-D magnetostatic model the cell's Maxwell H_z is
             // -Ms m_z - H_stat,z of the stage state (:3793-3804; the
             // sublattice terms are zero in a ferromagnetic cell)
-            if (P.mag1d_em) Hz = Hz + (-R(1.) * mat.Ms * mzc - io.Hstat.c[2][c]);
+            if (P.mag1d_em) Hz = Hz + (-R(1.) * mat.Ms * mzc - hs[2]);
             else Hz = Hz + (io.H_in.c[2][hz0] + io.H_in.c[2][hz1]) / R(2.);
         }
 
@@ -229,15 +241,6 @@ __global__ void __launch_bounds__(256, is_mixed<R>::value ? GF_LLG_MINB_F32 : GF
         dmx = precess * px + mat.alpha_precess * qx;
         dmy = precess * py + mat.alpha_precess * qy;
         dmz = precess * pz + mat.alpha_precess * qz;
-    }
-    // RK operands of the three components, loaded before the first store
-    R mx0[3], ma[3], mcm[3];
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-        mx0[a] = io.m_x.c[a][c];
-        ma[a] = (S > 0) ? io.m_acc.c[a][c] : R(0.);
-        mcm[a] = R(0.);
-        if constexpr (is_mixed<R>::value) { if (S == 3) mcm[a] = io.m_cmp.c[a][c]; }
     }
     if (P.em_fromM || P.spin) { io.dm.c[0][c] = dmx; io.dm.c[1][c] = dmy; io.dm.c[2][c] = dmz; }
 
