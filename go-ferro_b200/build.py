@@ -4,8 +4,11 @@
 
 Two CUDA translation units: gf_engine.cu (the FP64 parity kernels, the host
 engine and the C ABI) and gf_mixed.cu (the FP32 mixed-form stage kernels),
-both compiled with FMA contraction.  The library links cuFFT for the
-magnetostatic transforms.
+both compiled with FMA contraction.  Each unit is compiled whole: nvcc's
+-split-compile halves the build time, but which functions share a part then
+depends on the machine's load, and with it the register allocation of the
+column march (FP32 43 or 58 us per launch for one material).  The library links
+cuFFT for the magnetostatic transforms that gf_conv.cuh does not cover.
 """
 from __future__ import annotations
 
@@ -22,7 +25,7 @@ OUT = os.path.join(HERE, "libgoferro_b200.so")
 # (source, extra flags): each compiled to its own object, then linked
 UNITS = [("gf_engine.cu", ["-fmad=true"]), ("gf_mixed.cu", ["-fmad=true"]), ("gf_deck.cpp", [])]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-FLAGS = ["-O3", "-split-compile=8", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-O2", "-I" + os.path.join(ROOT, "include")]
+FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-O2", "-I" + os.path.join(ROOT, "include")]
 
 
 def nvcc() -> str:
