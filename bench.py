@@ -72,11 +72,10 @@ def alg_bytes_per_unit(kernel: str, info, mfe_frac: float = 0.0, mixed: bool = F
     D = 4.0 if mixed else 8.0
     comp = 0.5 if mixed else 0.0
     if kernel == "k_elastic":
-        # tiled stress-divergence kernel: u_in, m and p for the eigenstrain,
-        # material ids; writes the divergence and the crystal-frame strain of
-        # magnetic/ferroelectric cells
+        # stress-divergence kernel: u_in, m and p for the eigenstrain, material
+        # ids; writes the divergence and the crystal-frame strain of magnetic cells
         reads = 3 + 3 * info.fm + 3 * info.fe
-        writes = 3 + 6 * mfe_frac
+        writes = 3 + (6 * mfe_frac if info.fm else 0)
         return (reads + writes) * D + 1
     if kernel == "k_elastic_rk":
         # divergence, force_store, v_x, v_in, u_x (stages 1-3), v/u accumulators
@@ -89,7 +88,9 @@ def alg_bytes_per_unit(kernel: str, info, mfe_frac: float = 0.0, mixed: bool = F
         writes = 3 * 0.75 + 3 + 3 * info.em
         return (reads + writes + comp * 3) * D + 1
     if kernel == "k_fe":
-        reads = 3 + 3 + 3 * 0.75 + 3 + 3 + 3 * 0.75 + 6 + 6 + 3 + 3 * info.em
+        # p, q and u of the stage, step values, accumulators, E; the strain is
+        # formed from u
+        reads = 3 + 3 + 6 * 0.75 + 6 * 0.75 + 3 * info.elastic + 3 * info.em
         writes = 3 * 0.75 * 2 + 3 * 2
         return (reads + writes + comp * 6) * D + 1
     if kernel == "k_em_fused":
@@ -97,6 +98,18 @@ def alg_bytes_per_unit(kernel: str, info, mfe_frac: float = 0.0, mixed: bool = F
         # step value, accumulator read/write and stage output; dM/dt and dP/dt
         per_comp = 1 + 0.75 + 0.75 + 0.75 + 1 + comp
         return (6 * per_comp + 3 * info.fm + 3 * info.fe) * D + 1
+    if kernel in ("k_yee_E", "k_yee_H"):
+        # one of the two fields: its three components, the other field's three
+        # stage components, dP/dt (E) or dM/dt (H)
+        per_comp = 1 + 0.75 + 0.75 + 0.75 + 1 + comp
+        return (3 * per_comp + 3 + 3 * (info.fe if kernel == "k_yee_E" else info.fm)) * D + 0.5
+    if kernel in ("k_conv_fwd", "k_conv_inv"):
+        # three fields and their half spectra
+        return 6 * D
+    if kernel == "k_conv_x":
+        # the half spectra in and out, and the tensor's (six real in FP32,
+        # nine complex in FP64)
+        return (6 + (3 if mixed else 9)) * D
     return float("nan")
 
 
