@@ -138,3 +138,18 @@ fwrite(a.data(),8,n,stdout);fwrite(k.data(),16,h,stdout);fwrite(b.data(),8,n,std
     ref = np.fft.rfftn(a)
     assert np.max(np.abs(k - ref)) < 1e-12 * np.max(np.abs(ref))
     assert np.max(np.abs(b / n - a)) < 1e-14
+
+
+def test_smoke_has_reference_traces_without_the_oracle(gf, tmp_path):
+    import __graft_entry__
+
+    class NoOracle:
+        @staticmethod
+        def available():
+            return False
+    cases = list(__graft_entry__._smoke_cases(gf, NoOracle, str(tmp_path)))
+    assert {c[-1] for c in cases} == {"golden trace"}
+    assert any(d.magnetostatics and not d.elastic for d, *_ in cases) and any(d.elastic and d.em for d, *_ in cases)
+    for deck, ddir, probe, steps, ref, _ in cases:
+        assert ref.shape == (steps + 1, 22) and np.all(np.isfinite(ref)) and np.any(ref[:, 1] != 0.0)
+        assert os.path.exists(os.path.join(ddir, "system_setting.in")) and (probe is None) == (not deck.em)
