@@ -482,10 +482,11 @@ inline size_t conv_plane_smem(const ConvGeom& g) { return ((size_t)2 * g.plane +
 template <class R>
 inline size_t conv_x_smem(const ConvGeom& g) { return ((size_t)6 * g.g * g.nx + g.nx) * sizeof(Cx<R>); }
 
-// Geometry for a grid, or false when the transforms do not cover it (another
-// prime factor, or buffers beyond the shared memory of a block).
+// Geometry for a grid on a device of `sms` SMs, or false when the transforms
+// do not cover it (another prime factor, or buffers beyond the shared memory
+// of a block).
 template <class R>
-inline bool conv_geom(int nx, int ny, int nz, ConvGeom& g) {
+inline bool conv_geom(int nx, int ny, int nz, int sms, ConvGeom& g) {
     g = ConvGeom{};
     g.nx = nx; g.ny = ny; g.nz = nz; g.nzc = nz / 2 + 1;
     g.n = (long)nx * ny * nz;
@@ -499,12 +500,16 @@ inline bool conv_geom(int nx, int ny, int nz, ConvGeom& g) {
     if (conv_plane_smem<R>(g) > kConvMaxSmem) return false;
     g.dpairs = conv_div(g.pairs); g.dnz = conv_div(nz); g.dnzc = conv_div(g.nzc);
     // columns per block: 128-byte rows where two such blocks fit on an SM,
-    // fewer (never below 32 bytes) for long x; at least two blocks per SM of
-    // columns keep small films spread over the chip
+    // fewer (never below 32 bytes) for long x, and fewer on films whose blocks
+    // would be less than three for two SMs: between one and 1.5 per SM some
+    // SMs run two of the long blocks while the others wait (FP32 ms per step,
+    // at least 1 / 1.5 / 2 per SM: 108x120x24 0.154 / 0.148 / 0.149, 72x100x48
+    // 0.171 / 0.162 / 0.162; FP64 120x90x20 0.149 / 0.146 / 0.161, whose
+    // 32-byte rows cost more than they spread)
     int c = 128 / (int)sizeof(Cx<R>);
     const int least = 32 / (int)sizeof(Cx<R>);
     auto bytes = [&](int v) { return ((size_t)6 * v + 1) * nx * sizeof(Cx<R>); };
-    while (c > least && (bytes(c) > 100 * 1024 || (long)((g.cols + c - 1) / c) < 148)) c /= 2;
+    while (c > least && (bytes(c) > 100 * 1024 || 2l * ((g.cols + c - 1) / c) < 3l * sms)) c /= 2;
     if (bytes(c) > kConvMaxSmem) return false;
     g.g = c;
     g.groups = (g.cols + c - 1) / c;

@@ -1605,9 +1605,11 @@ int setup_demag(gf_engine* eng) {
     // the engine's own transforms where a stage solves for the field; a
     // field frozen at set-up (Maxwell runs) keeps cuFFT and, in FP64, the
     // reference's nine spectra
+    int sms = 1;
+    GF_CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, eng->device));
     eng->conv = eng->demag_per_stage &&
-                (eng->mixed ? conv_geom<float>(P.nx, P.ny, P.nz, eng->cg) && conv_pays<float>(eng->cg, d.elastodynamics)
-                            : conv_geom<double>(P.nx, P.ny, P.nz, eng->cg) && conv_pays<double>(eng->cg, d.elastodynamics));
+                (eng->mixed ? conv_geom<float>(P.nx, P.ny, P.nz, sms, eng->cg) && conv_pays<float>(eng->cg, d.elastodynamics)
+                            : conv_geom<double>(P.nx, P.ny, P.nz, sms, eng->cg) && conv_pays<double>(eng->cg, d.elastodynamics));
     if (eng->conv) {
         // k_conv_fwd forms Ms m itself: the LLG kernel writes m only
         eng->demag_src_fused = false;

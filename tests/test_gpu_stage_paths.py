@@ -186,10 +186,11 @@ def test_yee_update_equals_the_general_one(gf, name, precision):
 
 
 # sides with the transforms' radices 8, 4, 2, 3, 5 and their products, odd
-# ones, a single plane, row or layer, and (49, 22, 250) three that cuFFT keeps
+# ones, a single plane, row or layer, (49, 22, 250) three that cuFFT keeps, and
+# one whose x blocks take 8 columns with a remainder
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
 @pytest.mark.parametrize("shape", [(8, 6, 4), (5, 3, 2), (64, 16, 8), (30, 18, 10), (24, 45, 9), (128, 5, 3), (4, 4, 1), (1, 16, 6),
-                                   (20, 1, 5), (90, 2, 15), (49, 6, 4), (6, 22, 4), (250, 3, 2)])
+                                   (20, 1, 5), (90, 2, 15), (49, 6, 4), (6, 22, 4), (250, 3, 2), (6, 135, 27)])
 def test_stage_convolution_matches_the_restatement(gf, shape, precision):
     from oracle import restate_fm
     nx, ny, nz = shape
@@ -250,3 +251,17 @@ def test_adjoint_of_a_layered_film_matches_finite_differences(gf, tmp_path):
     gw32, ga32, _ = _grads(gf, tmp_path, d, steps, nw, wave0, alpha0, False, precision="mixed")
     assert np.max(np.abs(gw32 - gw)) <= 1e-3 * np.max(np.abs(gw))
     assert np.max(np.abs(ga32 - ga)) <= 1e-3 * np.max(np.abs(ga))
+
+
+def test_stage_convolution_of_the_widest_blocks(gf):
+    """x blocks of 16 columns with a remainder (FP32) against the FP64
+    form, whose blocks take 8."""
+    shape = (50, 216, 32)
+    d = gf.decks.preset_fm_demag(nx=shape[0], ny=shape[1], nz=shape[2], steps=10)
+    d.m0 = _unit(np.random.default_rng(43), shape)
+    H = {}
+    for precision in ("fp64", "mixed"):
+        with gf.Engine.from_params(d, device=0, precision=precision) as e:
+            H[precision] = e.download("Hstat")
+    assert np.linalg.norm(H["mixed"] - H["fp64"]) <= 3e-6 * np.linalg.norm(H["fp64"])
+
