@@ -518,19 +518,51 @@ inline bool conv_geom(int nx, int ny, int nz, int sms, ConvGeom& g) {
     return (long)g.plane < (1l << 20) && (long)3 * c * nx < (1l << 20) && (long)ny * nz < (1l << 20);
 }
 
-// Where the engine's transforms beat cuFFT's (ms per step, own / cuFFT).  A
-// film of ferromagnets alone: 36x128x5 0.073 / 0.099 FP32 and 0.076 / 0.103
-// FP64, 120x90x20 0.128 / 0.137 and 0.164 / 0.179, 128x128x32 0.196 / 0.213
-// and 0.312 / 0.339, but 192x192x24 0.321 / 0.301 and 0.539 / 0.537, 250x150x8
-// (an x of four passes) 0.168 / 0.172 and 0.280 / 0.263, 320x90x12 0.197 /
-// 0.196 and 0.305 / 0.282.  With elastodynamics the convolution runs beside
-// the elastic kernels and gains more from its few launches (ms per adjoint
-// pass: 250x150x20 17.0 / 17.4 and 25.5 / 25.5, 192x192x24 17.9 / 18.7 and
-// 26.6 / 28.1, 256x256x32 35.9 / 37.3 and 63.2 / 56.9).
+// plane blocks that fit on an SM by their shared memory
 template <class R>
-inline bool conv_pays(const ConvGeom& g, bool elastic) {
-    if (elastic) return sizeof(R) == 4 || g.n <= (1l << 20);
-    return g.n <= (1l << 19) && g.nx <= 256 && g.lx.np <= 3;
+inline int conv_plane_fit(const ConvGeom& g) { return (int)((size_t)227 * 1024 / (conv_plane_smem<R>(g) + 1024)); }
+
+// Where the engine's transforms beat cuFFT's in a stage, with or without
+// elastodynamics (the convolution follows the join of a stage's branches, so
+// it runs alone in both).  ms per step, own / cuFFT, FP32 and FP64, of films
+// of ferromagnets alone:
+//  * films up to 2^19 cells: 32x32x8 0.063 / 0.078 and 0.065 / 0.088, 64x64x16
+//    0.075 / 0.088 and 0.082 / 0.109, 120x90x20 0.120 / 0.126 and 0.150 /
+//    0.164, 128x128x32 0.189 / 0.204 and 0.284 / 0.313; beyond, 192x192x24
+//    0.320 / 0.299 and 0.530 / 0.537;
+//  * x in three passes of at most 256 points (an x block of four passes or of
+//    two per SM is long): 250x150x8 0.173 / 0.165 and 0.276 / 0.264, 512x64x8
+//    0.168 / 0.137 and 0.259 / 0.205;
+//  * planes that leave an SM three blocks in FP32, two in FP64, or that are all
+//    resident at once: 48x320x32 0.196 / 0.223 and 0.277 / 0.328, but 64x256x32
+//    (FP64, 192 blocks at one per SM) 0.358 / 0.307;
+//  * planes of more than 2048 points only where there is about one per SM:
+//    18x256x18 0.106 / 0.099 and 0.124 / 0.117, 24x384x32 0.182 / 0.170 and
+//    0.232 / 0.220, 24x200x50 0.170 / 0.147 and 0.216 / 0.199;
+//  * FP32: y of four passes only up to 2^17 cells: 90x135x8 0.095 / 0.109, but
+//    100x300x15 0.200 / 0.176 (FP64 0.331 / 0.352).
+// With elastodynamics the same lines hold: 90x120x40 0.284 / 0.294 and 0.423 /
+// 0.443, but 192x192x24 0.500 / 0.483 and 0.824 / 0.812.  Slower inside the
+// lines: FP32 108x120x24 0.148 / 0.145, FP64 240x90x24 0.307 / 0.302.
+template <class R>
+inline bool conv_pays(const ConvGeom& g, int sms) {
+    constexpr bool f32 = sizeof(R) == 4;
+    const int fit = conv_plane_fit<R>(g);
+    const long blocks = 3l * g.nx;
+    return g.n <= (1l << 19) && g.nx <= 256 && g.lx.np <= 3 && (fit >= (f32 ? 3 : 2) || blocks <= (long)fit * sms) &&
+           (g.plane <= 2048 || 10 * blocks >= 9l * sms) && (!f32 || g.ly.np <= 3 || g.n <= (1l << 17));
+}
+
+// The same for the discrete adjoint, which launches its stages one by one:
+// three launches in place of cuFFT's eight to twelve gain more there.  ms per
+// step of a forward and backward run of magnetoelastic films, own / cuFFT,
+// FP32 and FP64: 32x32x8 0.62 / 0.79 and 0.60 / 0.80, 108x120x24 1.30 / 1.39
+// and 1.52 / 1.72, 192x192x24 2.18 / 2.32 and 3.31 / 3.47, FP32 256x256x32 4.35
+// / 4.50; beyond the lines 512x512x8 4.90 / 4.78 and 8.3 / 7.7, FP64 256x256x32
+// 7.70 / 6.85, one plane block per SM (27x384x45 FP32) 1.86 / 1.82.
+template <class R>
+inline bool adj_conv_pays(const ConvGeom& g) {
+    return g.n <= (sizeof(R) == 4 ? (1l << 21) : (1l << 20)) && g.nx <= 256 && conv_plane_fit<R>(g) >= (sizeof(R) == 4 ? 2 : 1);
 }
 
 }  // namespace gf

@@ -137,7 +137,7 @@ struct gf_engine {
     ColGeom el_geom = {};
     // the per-stage magnetostatic convolution by the engine's own transforms
     // (gf_conv.cuh): geometry and twiddles
-    bool conv = false;
+    bool conv = false, cg_ok = false;      // the stages use it; the transforms cover the grid
     ConvGeom cg = {};
     void* conv_tw = nullptr;
     double* liao_hist = nullptr; double* liao_last = nullptr;
@@ -1535,19 +1535,11 @@ std::shared_ptr<const std::vector<double>> newell_tables(const Params& P) {
     return last;
 }
 
-// buffers of the convolution: M_k, H (3n, H_stat is a view of it), the
-// twiddles of the three lengths, and the tensor's spectra from the host's FP64
-// tables (a temporary cuFFT plan; FP32 keeps the six real ones)
+// what the convolution kernels need beside M_k, H and the spectra: the
+// twiddles of the three lengths and the shared-memory opt-in
 template <class R>
-int conv_setup(gf_engine* eng) {
+int conv_kernels(gf_engine* eng) {
     const Params& P = eng->P;
-    const long n = P.n, nk = eng->cg.nk;
-    int dims[3] = {P.nx, P.ny, P.nz};
-    GF_TRY(dalloc(eng, reinterpret_cast<void**>(&eng->Mfft), sizeof(R) * 3 * (size_t)n));
-    GF_TRY(dalloc(eng, reinterpret_cast<void**>(&eng->Mk), sizeof(Cx<R>) * 3 * (size_t)nk));
-    if constexpr (is_mixed<R>::value) GF_TRY(dalloc(eng, reinterpret_cast<void**>(&eng->Nr), sizeof(float) * 6 * (size_t)nk));
-    else GF_TRY(dalloc_n(eng, &eng->Nk, (size_t)9 * nk));
-    for (int a = 0; a < 3; a++) eng->Hstat[a] = reinterpret_cast<double*>(reinterpret_cast<R*>(eng->Mfft) + (size_t)a * n);
     std::vector<Cx<R>> tw;
     for (int len : {P.nx, P.ny, P.nz})
         for (int k = 0; k < len; k++) {
@@ -1558,6 +1550,23 @@ int conv_setup(gf_engine* eng) {
     GF_CU(cudaMemcpy(eng->conv_tw, tw.data(), sizeof(Cx<R>) * tw.size(), cudaMemcpyHostToDevice));
     GF_TRY(conv_attr<R>(eng));
     if (eng->mixed) GF_TRY(gf_mixed_conv_attr(eng));
+    return GF_OK;
+}
+
+// buffers of the convolution: M_k, H (3n, H_stat is a view of it), and the
+// tensor's spectra from the host's FP64 tables (a temporary cuFFT plan; FP32
+// keeps the six real ones)
+template <class R>
+int conv_setup(gf_engine* eng) {
+    const Params& P = eng->P;
+    const long n = P.n, nk = eng->cg.nk;
+    int dims[3] = {P.nx, P.ny, P.nz};
+    GF_TRY(dalloc(eng, reinterpret_cast<void**>(&eng->Mfft), sizeof(R) * 3 * (size_t)n));
+    GF_TRY(dalloc(eng, reinterpret_cast<void**>(&eng->Mk), sizeof(Cx<R>) * 3 * (size_t)nk));
+    if constexpr (is_mixed<R>::value) GF_TRY(dalloc(eng, reinterpret_cast<void**>(&eng->Nr), sizeof(float) * 6 * (size_t)nk));
+    else GF_TRY(dalloc_n(eng, &eng->Nk, (size_t)9 * nk));
+    for (int a = 0; a < 3; a++) eng->Hstat[a] = reinterpret_cast<double*>(reinterpret_cast<R*>(eng->Mfft) + (size_t)a * n);
+    GF_TRY(conv_kernels<R>(eng));
     const std::shared_ptr<const std::vector<double>> host_tab = newell_tables(P);
     double* tab = nullptr;
     cufftDoubleComplex* nk64 = nullptr;
@@ -1607,9 +1616,8 @@ int setup_demag(gf_engine* eng) {
     // reference's nine spectra
     int sms = 1;
     GF_CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, eng->device));
-    eng->conv = eng->demag_per_stage &&
-                (eng->mixed ? conv_geom<float>(P.nx, P.ny, P.nz, sms, eng->cg) && conv_pays<float>(eng->cg, d.elastodynamics)
-                            : conv_geom<double>(P.nx, P.ny, P.nz, sms, eng->cg) && conv_pays<double>(eng->cg, d.elastodynamics));
+    eng->cg_ok = eng->mixed ? conv_geom<float>(P.nx, P.ny, P.nz, sms, eng->cg) : conv_geom<double>(P.nx, P.ny, P.nz, sms, eng->cg);
+    eng->conv = eng->demag_per_stage && eng->cg_ok && (eng->mixed ? conv_pays<float>(eng->cg, sms) : conv_pays<double>(eng->cg, sms));
     if (eng->conv) {
         // k_conv_fwd forms Ms m itself: the LLG kernel writes m only
         eng->demag_src_fused = false;
@@ -4353,6 +4361,7 @@ struct gf_adjoint {
     // trace and its cotangent stay FP64; every buffer below except abar,
     // wbar, trace and dldm holds elements of esz bytes
     bool f32 = false;
+    bool conv = false;               // magnetostatics by the engine's own transforms (adj_conv_pays)
     size_t esz = sizeof(double);
     std::vector<void*> allocs;
     void* am = nullptr;              // AdjMatT<R> per material
@@ -4459,7 +4468,7 @@ int adj_demag(gf_adjoint* a, F3T<R> y, F3T<R>& hd) {
     gf_engine* eng = a->eng;
     const Params& P = eng->P;
     if (eng->demag_mode != 0) { hd = v3c<R>(rp<R>(a->zero3), P.n); return GF_OK; }
-    if (eng->conv) {
+    if (a->conv) {
         hd = v3c<R>(rp<R>(eng->Mfft), P.n);
         return conv_solve<R>(eng, y, true, hd, false);
     }
@@ -4498,7 +4507,7 @@ int adj_demag_T(gf_adjoint* a, const R*& out) {
     const unsigned bn = blocks_for(P.n, kThreads);
     const long n21 = (long)P.nx * P.ny * (P.nz / 2 + 1);
     R* M3 = reinterpret_cast<R*>(eng->Mfft);
-    if (eng->conv) {
+    if (a->conv) {
         out = M3;
         return conv_solve<R>(eng, v3<R>(a->HBAR), false, v3c<R>(M3, P.n), false);
     }
@@ -5011,6 +5020,8 @@ int gf_adjoint_create(gf_engine* e, int n_wave, int checkpoint_every, gf_adjoint
     auto fail = [&](int rc) { gf_adjoint_destroy(a); return rc; };
     int rc = a->f32 ? adj_tables<float>(a) : adj_tables<double>(a);
     if (rc != GF_OK) return fail(rc);
+    a->conv = eng->conv || (eng->demag_mode == 0 && eng->cg_ok && (a->f32 ? adj_conv_pays<float>(eng->cg) : adj_conv_pays<double>(eng->cg)));
+    if (a->conv && !eng->conv_tw && (rc = a->f32 ? conv_kernels<float>(eng) : conv_kernels<double>(eng)) != GF_OK) return fail(rc);
     // per-cell damping, default the material's alpha
     const long n = P.n;
     if ((rc = adj_alloc(a, &a->alpha, (size_t)n)) != GF_OK) return fail(rc);

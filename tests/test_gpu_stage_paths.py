@@ -254,8 +254,8 @@ def test_adjoint_of_a_layered_film_matches_finite_differences(gf, tmp_path):
 
 
 def test_stage_convolution_of_the_widest_blocks(gf):
-    """x blocks of 16 columns with a remainder (FP32) against the FP64
-    form, whose blocks take 8."""
+    """x blocks of 16 columns with a remainder (FP32) against cuFFT, which the
+    FP64 form keeps for planes of this size."""
     shape = (50, 216, 32)
     d = gf.decks.preset_fm_demag(nx=shape[0], ny=shape[1], nz=shape[2], steps=10)
     d.m0 = _unit(np.random.default_rng(43), shape)
@@ -265,3 +265,20 @@ def test_stage_convolution_of_the_widest_blocks(gf):
             H[precision] = e.download("Hstat")
     assert np.linalg.norm(H["mixed"] - H["fp64"]) <= 3e-6 * np.linalg.norm(H["fp64"])
 
+
+# x of four passes, which the engine leaves to cuFFT and the adjoint takes by
+# its own transforms
+@pytest.mark.parametrize("shape", [(81, 6, 6), (250, 8, 5)])
+def test_adjoint_transforms_match_the_engine(gf, shape):
+    D = gf.decks
+    d = D.preset_fm_demag(nx=shape[0], ny=shape[1], nz=shape[2], steps=6)
+    d.Hext_table = None
+    d.Hext_stat = (0.0, 0.0, 1.0 / D.MU0)
+    d.m0 = D.tilt_m0(shape, 41, d.material_cell(), 20.0)
+    for precision, tol in (("fp64", 1e-12), ("mixed", 1e-6)):
+        with gf.Engine.from_params(d, device=0, precision=precision) as e:
+            with gf.Adjoint(e, n_wave=4, checkpoint_every=3) as a:
+                a.forward(6)
+                m = a.final_m()
+            e.advance(6)
+            assert np.max(np.abs(m - e.download("m"))) <= tol
