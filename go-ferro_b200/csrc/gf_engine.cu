@@ -218,7 +218,7 @@ int gf_mixed_elastic_setup(gf_engine* eng, int smem, int* per_sm);   // shared-m
 int gf_mixed_conv_attr(gf_engine* eng);                                 // shared-memory opt-in of the convolution kernels
 int gf_mixed_col_setup(gf_engine* eng);                                 // the same for k_elastic_col, and its tile
 int gf_mixed_time_tile(gf_engine* eng, int reps, float* ms);          // stage-1 elastic tile, mean ms per launch
-int gf_mixed_adj_elastic(gf_engine* eng, int s, int rk, const StageIOT<float>& io);  // adjoint: FP32 elastic tile / RK of stage s
+int gf_mixed_adj_elastic(gf_engine* eng, int s, int rk, const StageIOT<float>& io);  // adjoint: FP32 stress divergence / RK of stage s
 int gf_mixed_batch_attr(size_t smem);                                   // shared-memory opt-in of the batch phase kernels
 int gf_mixed_batch_persistent_blocks(size_t smem, int* blocks);          // co-resident blocks of k_batch_persistent
 int gf_mixed_batch_persistent(const BatchInst* insts, int ninst, const BatchItem* A, int nA, const BatchItem* L, int nB, int nC,
@@ -1374,10 +1374,9 @@ int gf_mixed_col_setup(gf_engine* eng) { return col_setup<float>(eng); }
 
 int gf_mixed_time_tile(gf_engine* eng, int reps, float* ms) { return time_tile_t<float>(eng, reps, ms); }
 
-// the FP32 elastic tile (rk = 0) or RK update (rk = 1) of stage s on the
-// discrete adjoint's buffers (io built by the adjoint), with the engine's
-// launch shapes; the tile stages by cp.async (no tensor maps over the
-// adjoint's buffers)
+// the FP32 stress divergence (rk = 0; adjoint decks are on col_path) or RK
+// update (rk = 1) of stage s on the discrete adjoint's buffers (io built by
+// the adjoint), with the engine's launch shapes
 namespace {
 template <int S>
 int adj_elastic_f32(gf_engine* eng, int rk, const StageIOT<float>& io) {
@@ -1389,21 +1388,7 @@ int adj_elastic_f32(gf_engine* eng, int rk, const StageIOT<float>& io) {
         GF_CU(launch(k_elastic_rk<S, float>, dim3(blocks_for(P.n, 2 * kThreads)), dim3(kThreads), 0, eng->stream, Pa, io));
         return GF_OK;
     }
-    if (eng->el_col) {
-        GF_CU(col_launch<float>(eng, io, eng->stream, false));
-        return GF_OK;
-    }
-    ETileMaps tm;
-    std::memset(&tm, 0, sizeof(tm));
-    tm.err = eng->tma_err;
-    const dim3 grid((P.nz + etile::TK - 1) / etile::TK, (P.ny + etile::TJ - 1) / etile::TJ,
-                    (P.nx + eng->el_chunk - 1) / eng->el_chunk);
-    if (eng->el_cubic)
-        GF_CU(launch_tiled(k_elastic_tile<S, true, float>, grid, dim3(etile::NT), eng->el_smem, eng->stream, P, io,
-                           eng->el_chunk, eng->el_nmat, tm));
-    else
-        GF_CU(launch_tiled(k_elastic_tile<S, false, float>, grid, dim3(etile::NT), eng->el_smem, eng->stream, P, io,
-                           eng->el_chunk, eng->el_nmat, tm));
+    GF_CU(col_launch<float>(eng, io, eng->stream, false));
     return GF_OK;
 }
 }  // namespace
@@ -4557,8 +4542,8 @@ StageIOT<R> adj_el_io(gf_adjoint* a, double* const* x, F3T<R> ym, F3T<R> yu, F3T
     return io;
 }
 
-// the engine's elastic tile (rk = 0) or RK update (rk = 1) of stage S on the
-// adjoint's buffers; FP32 through the mixed translation unit, so that the
+// the engine's stress divergence (rk = 0; adjoint decks are on col_path) or RK
+// update (rk = 1) of stage S on the adjoint's buffers; FP32 through the mixed translation unit, so that the
 // adjoint's forward run is the mixed engine's own elastic discretisation
 template <int S>
 int adj_el_kernel(gf_adjoint* a, int rk, const StageIOT<double>& io) {
@@ -4571,21 +4556,7 @@ int adj_el_kernel(gf_adjoint* a, int rk, const StageIOT<double>& io) {
         GF_CU(launch(k_elastic_rk<S, double>, dim3(blocks_for(P.n, kThreads)), dim3(kThreads), 0, eng->stream, Pa, io));
         return GF_OK;
     }
-    if (eng->el_col) {
-        GF_CU(col_launch<double>(eng, io, eng->stream, false));
-        return GF_OK;
-    }
-    ETileMaps tm;
-    std::memset(&tm, 0, sizeof(tm));
-    tm.err = eng->tma_err;
-    const dim3 grid((P.nz + etile::TK - 1) / etile::TK, (P.ny + etile::TJ - 1) / etile::TJ,
-                    (P.nx + eng->el_chunk - 1) / eng->el_chunk);
-    if (eng->el_cubic)
-        GF_CU(launch_tiled(k_elastic_tile<S, true, double>, grid, dim3(etile::NT), eng->el_smem, eng->stream, P, io,
-                           eng->el_chunk, eng->el_nmat, tm));
-    else
-        GF_CU(launch_tiled(k_elastic_tile<S, false, double>, grid, dim3(etile::NT), eng->el_smem, eng->stream, P, io,
-                           eng->el_chunk, eng->el_nmat, tm));
+    GF_CU(col_launch<double>(eng, io, eng->stream, false));
     return GF_OK;
 }
 template <class R>
