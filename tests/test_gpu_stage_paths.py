@@ -140,6 +140,23 @@ def test_column_march_equals_the_general_tile(gf, name, precision):
     _same(_run(gf, d, precision), _run(gf, g, precision), TOL[precision])
 
 
+# Isotropic stiffness, electrostriction and Landau coefficients: the physics
+# does not know the crystal frame, so a rotated one (strain, eigenstrain,
+# stiffness and polarisation go through the frame rotations, the stress through
+# the general tile) gives the run of the unrotated one.  The rotations add a few
+# roundings to each term, no cancellation: the tolerances above hold.
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_rotated_frame_of_an_isotropic_film_changes_nothing(gf, precision):
+    D = gf.decks
+    film = dataclasses.replace(D.pto(), c44=0.5 * (2.3e11 - 1.0e11), Q44=0.089 + 0.026, a11=7e7, a12=1.4e8,
+                               a111=2.6e8, a112=7.8e8, a123=1.56e9)
+    substrate = dataclasses.replace(D.ggg(), c44=0.5 * (2.86e11 - 1.16e11))
+    d = _moving(_fe(gf, 6, 15, 14, materials=[substrate, film], layers=[(4, 1), (8, 2), (2, 0)]), 47)
+    a = _run(gf, d, precision)
+    assert all(np.linalg.norm(a[f]) > 0.0 for f in ("p", "q", "u", "v", "Ex", "Hz"))
+    _same(_run(gf, dataclasses.replace(d, Tg2c=D.rotation(30.0, 20.0)), precision), a, TOL[precision])
+
+
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
 @pytest.mark.parametrize("shape", [(1, 5, 5), (9, 21, 13), (12, 33, 32)])
 @pytest.mark.parametrize("elastic", [True, False])
