@@ -270,12 +270,11 @@ static __global__ void k_batch_step_inc(const BatchInst* __restrict__ insts, int
     if (t < count) *insts[t].step = *insts[t].step + 1ull;
 }
 
-// shared memory of a phase-A block: the elastic tile's, or the Yee
-// kernel's two tables
+// shared memory of a phase-A block: the elastic tile's, the column march's or
+// the Yee kernel's two tables
 inline size_t batch_smem_bytes(int nmat) {
     const size_t em = kMaxMat * sizeof(EmMat<float>) + kEmMaxCls * sizeof(EmCls<float>);
-    const size_t tile = etile::smem_bytes<float>(nmat);
-    return tile > em ? tile : em;
+    return std::max({etile::smem_bytes<float>(nmat), col_smem_bytes<float>(kColBatchThreads, nmat), em});
 }
 
 }  // namespace gf

@@ -3646,7 +3646,7 @@ const char* gf_version(void) { return "goferro_b200 0.2 (FP64 parity form, FP32 
 // ===========================================================================
 struct gf_batch {
     std::vector<gf_engine*> engs;
-    int device = 0;
+    int device = 0, sms = 1;
     cudaStream_t stream = nullptr;
     cudaEvent_t fork = nullptr;
     std::vector<cudaEvent_t> join;
@@ -3730,11 +3730,12 @@ std::string batch_phase_blocker(const gf_engine* e) {
     return "";
 }
 
-// column tile of engine e's work items: at most a batch block's threads
-ColGeom batch_geom(const gf_engine* e, int chunk) {
+// column tile of engine e's work items: at most a batch block's threads, on
+// the blocks per SM of the tile items' kernel, which the items of all engines share
+ColGeom batch_geom(const gf_batch* b, const gf_engine* e, int chunk) {
     if (!e->el_col) return ColGeom{};
-    // the items of all engines share an SM's slots
-    return col_geom<float>(e->P, kColBatchThreads, 148, [](int) { return 148L * 3; }, std::min(chunk, (int)e->P.nx));
+    return col_geom<float>(e->P, kColBatchThreads, b->sms, [b](int) { return (long)b->sms * GF_BATCH_TILE_MINB; },
+                           std::min(chunk, (int)e->P.nx));
 }
 
 // the work items of every engine at elastic x-chunk ch[i]: phase A's tile,
@@ -3751,7 +3752,7 @@ void batch_items(const gf_batch* b, const std::vector<int>& ch, std::vector<Batc
         const long nx = P.nx, ny = P.ny, nz = P.nz;
         if (P.elastic) {
             const gf_engine* e = b->engs[i];
-            const ColGeom g = batch_geom(e, ch[i]);
+            const ColGeom g = batch_geom(b, e, ch[i]);
             const int gx = e->el_col ? g.tk : (P.nz + etile::TK - 1) / etile::TK;
             const int gy = e->el_col ? g.tj : (P.ny + etile::TJ - 1) / etile::TJ;
             const int gz = (P.nx + ch[i] - 1) / ch[i];
@@ -3806,7 +3807,7 @@ int batch_upload(gf_batch* b, const std::vector<int>& ch) {
         t.uni = e->uni && (e->um_f.flags & MF_FE) ? 1 : 0;
         t.um = e->um_f;
         t.el_pm = col_pm(e);
-        t.geom = batch_geom(e, ch[i]);
+        t.geom = batch_geom(b, e, ch[i]);
         t.step = e->step_ctr;
     }
     std::vector<BatchItem> A, At, Ae, Af, B, C, D;
@@ -4155,6 +4156,7 @@ int gf_batch_create_ex(gf_engine* const* engines, int count, int autotune, int m
     }
     auto fail = [&](int rc) { g_create_err = b->err; gf_batch_destroy(b); return rc; };
     if (cudaSetDevice(b->device) != cudaSuccess) { b->err = "cudaSetDevice"; return fail(GF_ECUDA); }
+    if (cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, b->device) != cudaSuccess) { b->err = "device attribute"; return fail(GF_ECUDA); }
     if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess) { b->err = "stream"; return fail(GF_ECUDA); }
     if (cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming) != cudaSuccess) { b->err = "event"; return fail(GF_ECUDA); }
     b->join.assign(b->engs.size(), nullptr);
