@@ -214,12 +214,12 @@ struct gf_engine {
 // functions are its interface.
 int gf_mixed_enqueue_step(gf_engine* eng, int parity);                 // kernels of one step, mixed form
 int gf_mixed_enqueue_stage(gf_engine* eng, int parity, int s);         // kernels of stage s (0..3), mixed form
-int gf_mixed_elastic_setup(gf_engine* eng, int smem, int* per_sm);   // shared-memory opt-in, occupancy
+int gf_mixed_elastic_setup(gf_engine* eng, int* per_sm);             // shared-memory opt-in, occupancy
 int gf_mixed_conv_attr(gf_engine* eng);                                 // shared-memory opt-in of the convolution kernels
 int gf_mixed_col_setup(gf_engine* eng);                                 // the same for k_elastic_col, and its tile
 int gf_mixed_time_tile(gf_engine* eng, int reps, float* ms);          // stage-1 elastic tile, mean ms per launch
 int gf_mixed_adj_elastic(gf_engine* eng, int s, int rk, const StageIOT<float>& io);  // adjoint: FP32 stress divergence / RK of stage s
-int gf_mixed_batch_attr(size_t smem);                                   // shared-memory opt-in of the batch phase kernels
+int gf_mixed_batch_attr();                                              // shared-memory opt-in of the batch phase kernels
 int gf_mixed_batch_persistent_blocks(size_t smem, int* blocks);          // co-resident blocks of k_batch_persistent
 int gf_mixed_batch_persistent(const BatchInst* insts, int ninst, const BatchItem* A, int nA, const BatchItem* L, int nB, int nC,
                               int nD, int parity, size_t smem, unsigned* err, unsigned* bar, int blocks, cudaStream_t st);
@@ -849,19 +849,17 @@ void build_io_mixed(gf_engine* eng) {
 // ---------------------------------------------------------------------------
 // one RK4 step: kernel sequence in the reference's data order
 // ---------------------------------------------------------------------------
-// Shared-memory opt-in and the x-chunk of the tiled elastic kernel.  A
-// block of `L` planes costs L+2 plane passes (one halo plane each side), so
-// the chunk count minimises waves x (L+2) over the blocks that fit at once.
+// Shared-memory opt-in of the tiled elastic kernel.  A function's attribute is
+// the process's: set it for the most materials a deck can have, so that engines
+// with fewer do not lower it.
 template <class R>
-int set_elastic_smem(gf_engine* eng, int smem) {
-    GF_CU(cudaFuncSetAttribute(k_elastic_tile<0, true, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    GF_CU(cudaFuncSetAttribute(k_elastic_tile<1, true, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    GF_CU(cudaFuncSetAttribute(k_elastic_tile<2, true, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    GF_CU(cudaFuncSetAttribute(k_elastic_tile<3, true, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    GF_CU(cudaFuncSetAttribute(k_elastic_tile<0, false, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    GF_CU(cudaFuncSetAttribute(k_elastic_tile<1, false, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    GF_CU(cudaFuncSetAttribute(k_elastic_tile<2, false, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    GF_CU(cudaFuncSetAttribute(k_elastic_tile<3, false, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+int set_elastic_smem(gf_engine* eng) {
+    const int smem = (int)etile::smem_bytes<R>(kMaxMat);
+    auto set = [&](auto k) { return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); };
+    GF_CU(set(k_elastic_tile<0, true, R>)); GF_CU(set(k_elastic_tile<1, true, R>));
+    GF_CU(set(k_elastic_tile<2, true, R>)); GF_CU(set(k_elastic_tile<3, true, R>));
+    GF_CU(set(k_elastic_tile<0, false, R>)); GF_CU(set(k_elastic_tile<1, false, R>));
+    GF_CU(set(k_elastic_tile<2, false, R>)); GF_CU(set(k_elastic_tile<3, false, R>));
     return GF_OK;
 }
 
@@ -948,7 +946,6 @@ int setup_elastic_tile(gf_engine* eng) {
     const Params& P = eng->P;
     eng->el_nmat = (int)eng->deck.mats.size();
     eng->el_smem = eng->mixed ? etile::smem_bytes<float>(eng->el_nmat) : etile::smem_bytes<double>(eng->el_nmat);
-    const int smem = (int)eng->el_smem;
     eng->el_cubic = true;
     for (const Material& m : eng->deck.mats)
         for (int a = 0; a < 6; a++)
@@ -960,9 +957,9 @@ int setup_elastic_tile(gf_engine* eng) {
     }
     int per_sm = 1, sms = 1;
     if (eng->mixed) {
-        GF_TRY(gf_mixed_elastic_setup(eng, smem, &per_sm));
+        GF_TRY(gf_mixed_elastic_setup(eng, &per_sm));
     } else {
-        GF_TRY(set_elastic_smem<double>(eng, smem));
+        GF_TRY(set_elastic_smem<double>(eng));
         GF_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_elastic_tile<1, false, double>, etile::NT, eng->el_smem));
     }
     GF_CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, eng->device));
@@ -978,6 +975,8 @@ int setup_elastic_tile(gf_engine* eng) {
     // did the FP32 magnetoelastic film, whose LLG kernel waits for it, 0.878
     // -> 1.014 ms)
     if (eng->mixed && P.fe && !(P.fm || P.afm)) slots = std::max<long>(1, slots * 3 / 5);
+    // a block of L planes costs L+2 plane passes (one halo plane each side): the
+    // chunk count minimises waves x (L+2) over the blocks that fit at once
     const long tiles = (long)((P.nz + etile::TK - 1) / etile::TK) * ((P.ny + etile::TJ - 1) / etile::TJ);
     long best_cost = -1;
     for (long c = 1; c <= P.nx; c++) {
@@ -1363,9 +1362,9 @@ int enqueue_stage_t(gf_engine* eng, int parity, int s) {
 int gf_mixed_enqueue_step(gf_engine* eng, int parity) { return enqueue_step_t<float>(eng, parity); }
 int gf_mixed_enqueue_stage(gf_engine* eng, int parity, int s) { return enqueue_stage_t<float>(eng, parity, s); }
 
-int gf_mixed_elastic_setup(gf_engine* eng, int smem, int* per_sm) {
-    GF_TRY(set_elastic_smem<float>(eng, smem));
-    GF_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k_elastic_tile<1, false, float>, etile::NT, (size_t)smem));
+int gf_mixed_elastic_setup(gf_engine* eng, int* per_sm) {
+    GF_TRY(set_elastic_smem<float>(eng));
+    GF_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k_elastic_tile<1, false, float>, etile::NT, eng->el_smem));
     return GF_OK;
 }
 
@@ -1393,8 +1392,8 @@ int adj_elastic_f32(gf_engine* eng, int rk, const StageIOT<float>& io) {
 }
 }  // namespace
 
-int gf_mixed_batch_attr(size_t smem) {
-    const int b = (int)smem;
+int gf_mixed_batch_attr() {
+    const int b = (int)batch_smem_bytes(kMaxMat);     // as in set_elastic_smem
     cudaError_t e = cudaSuccess;
     auto set = [&](auto k) { if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, b); };
     set(k_batch_phase<0, 0>); set(k_batch_phase<1, 0>); set(k_batch_phase<2, 0>); set(k_batch_phase<3, 0>);
@@ -4180,7 +4179,7 @@ int gf_batch_create_ex(gf_engine* const* engines, int count, int autotune, int m
         int nmat = 1;
         for (gf_engine* e : b->engs) nmat = std::max(nmat, (int)e->deck.mats.size());
         b->smem = batch_smem_bytes(nmat);
-        if (gf_mixed_batch_attr(b->smem) != GF_OK) { b->err = "batch kernels: shared-memory attribute"; return fail(GF_ECUDA); }
+        if (gf_mixed_batch_attr() != GF_OK) { b->err = "batch kernels: shared-memory attribute"; return fail(GF_ECUDA); }
         int rc = batch_tune_phases(b, autotune);
         if (rc != GF_OK) return fail(rc);
         if (cudaStreamSynchronize(b->stream) != cudaSuccess) { b->err = "batch tuning"; return fail(GF_ECUDA); }

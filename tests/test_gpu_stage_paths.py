@@ -158,6 +158,20 @@ def test_rotated_frame_of_an_isotropic_film_changes_nothing(gf, precision):
 
 
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_an_engine_of_fewer_materials_leaves_the_others_their_tile(gf, precision):
+    """The tile's shared-memory limit belongs to the process, not to the engine
+    created last (ny < nz: the general tile)."""
+    one = _moving(_fe(gf, 4, 8, 16), 53)
+    many = dataclasses.replace(one, materials=one.materials * 12)
+    want = _run(gf, one, precision, 1)
+    with gf.Engine.from_params(many, device=0, precision=precision) as e:
+        with gf.Engine.from_params(one, device=0, precision=precision):
+            e.advance(1)
+            got = e.download("u")
+    assert np.linalg.norm(got - want["u"]) <= TOL[precision] * np.linalg.norm(want["u"])
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
 @pytest.mark.parametrize("shape", [(1, 5, 5), (9, 21, 13), (12, 33, 32)])
 @pytest.mark.parametrize("elastic", [True, False])
 def test_tdgl_of_one_material_equals_two_alike(gf, shape, elastic, precision):
