@@ -964,17 +964,12 @@ int setup_elastic_tile(gf_engine* eng) {
     }
     GF_CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, eng->device));
     if (per_sm < 1) { eng->err = "elastic tile does not fit on an SM"; return GF_ECUDA; }
-    long slots = (long)per_sm * (sms > 0 ? sms : 1);
-    // In the mixed form without magnets the TDGL and Maxwell kernels do not
-    // wait for the tile and share the SMs with it: the tile's blocks are held
-    // to three fifths of the resident slots, which leaves them room (128^3
-    // ferroelectric FP32 step, ms, by planes per block and share of the
-    // slots: 16 / 86 % 1.355, 19 / 76 % 1.338, 22 / 65 % 1.327, 26 / 54 %
-    // 1.322, 32 / 43 % 1.351; the FP64 step, whose TDGL kernel waits for the
-    // tile, measured slower with the smaller share, 2.379 -> 2.395 ms, and so
-    // did the FP32 magnetoelastic film, whose LLG kernel waits for it, 0.878
-    // -> 1.014 ms)
-    if (eng->mixed && P.fe && !(P.fm || P.afm)) slots = std::max<long>(1, slots * 3 / 5);
+    // every slot, in both forms, also where the TDGL and Maxwell kernels run
+    // beside the tile (ferroelectric decks, ms per step with all / 86 / 60 % of
+    // the slots: FP32 128x96x128 0.921 / 0.980 / 1.212, rotated 128^3 1.317 /
+    // 1.305 / 1.392, rotated 75x61x37 0.222 / 0.224 / 0.260; FP64 1.557 / 1.628 /
+    // 1.607, 2.189 / 2.218 / 2.246, 0.294 / 0.296 / 0.363)
+    const long slots = (long)per_sm * (sms > 0 ? sms : 1);
     // a block of L planes costs L+2 plane passes (one halo plane each side): the
     // chunk count minimises waves x (L+2) over the blocks that fit at once
     const long tiles = (long)((P.nz + etile::TK - 1) / etile::TK) * ((P.ny + etile::TJ - 1) / etile::TJ);
