@@ -267,7 +267,7 @@ __global__ void __launch_bounds__(256) k_adj_vjp(Params P, const uint8_t* __rest
 
 // ---------------------------------------------------------------------------
 // Elastodynamic coupling (magnetoelastic decks).  Forward per stage s (the
-// engine's own k_elastic_tile and k_elastic_rk on the adjoint's buffers):
+// engine's own k_elastic_col and k_elastic_rk on the adjoint's buffers):
 //   f = div sigma(u_s, e0(m_s)),  e_s = cell strain of u_s (LLG field),
 //   k_u = dt v_s,  k_v = dens_dt f + md v_x + sd w_s (f - fs),
 // with v_x the step value, w = 1, 2, 2, 1 and fs the stage-1 force of the

@@ -3,7 +3,7 @@
 //
 // A stage of a ferroelectric + elastodynamics + FDTD engine is a few phases
 // whose kernels depend only on the phases before:
-//   A: elastic tile (stress divergence), TDGL, Yee update
+//   A: stress divergence (column march or general tile), TDGL, Yee update
 //   B: elastic RK update, the first Mur boundary of E  (read A's outputs)
 //   C: elastic boundary planes (after the RK update; none where the RK
 //      update applies them itself, Params::el_bc_fused), the second Mur

@@ -78,10 +78,12 @@ struct ColGeom {
 };
 // Threads of the per-engine kernel, and the blocks per SM its registers
 // allow: the column's state must not spill (us per launch on the 128^3
-// ferroelectric grid / the 128x128x96 film of several materials: FP64 384 x 1
+// ferroelectric grid / the 128x128x96 film of several materials, before the
+// tile shape was chosen by col_geom and the material by template: FP64 384 x 1
 // block, 168 registers, 72 / 80; 512 x 1, 128 registers, 86 / 127; 256 x 2,
 // 104 / 132; 256 x 3, 145 / 191.  FP32 384 x 2, 80 registers, 56 / 67; 256 x 3
-// 56 / 68; 512 x 2, 64 registers, 65 / 94; 256 x 4 65 / 89).
+// 56 / 68; 512 x 2, 64 registers, 65 / 94; 256 x 4 65 / 89.  Now 61 / 66 in FP64
+// and 43 / 50 in FP32; the general tile took 255 / 183 and 159 / 99).
 #ifndef GF_ECOL_T_F32
 #define GF_ECOL_T_F32 384
 #endif

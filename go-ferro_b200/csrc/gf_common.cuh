@@ -80,7 +80,7 @@ struct Params {
     int per_x, per_y, per_z;
     long n;
     double dx, dy, dz, dt;
-    double rdx, rdy, rdz, rdt;   // correctly rounded reciprocals (host 1./dx ...), for qdiv
+    double rdx, rdy, rdz, rdt;   // correctly rounded reciprocals (host 1./dx ...), for qdivR
     double dt_e0, mdt_mu0;       // dt / e0 and -dt / mu0, rounded as the reference does
     int rot;                 // if_OrientRotate
     double Tg2c[3][3], Tc2g[3][3];
@@ -174,8 +174,8 @@ __device__ __forceinline__ double qdiv(double x, double d, double rd) {
 }
 
 // Division by a run constant d in the stencils: a multiplication by its
-// rounded reciprocal (rd = RN(1/d), rdf in FP32), within one ulp of the
-// quotient.  qdiv's exact quotient costs five FP64 operations and a select
+// rounded reciprocal (rd = RN(1/d), rdf in FP32): two roundings, within two ulps
+// of the quotient.  qdiv's exact quotient costs five FP64 operations and a select
 // where this costs one, at up to 60 divisions per cell and stage (128^3
 // ferroelectric, FP64, us per launch with both this and contraction: elastic
 // tile 255 -> 230, Yee 152 -> 144, TDGL 134 -> 130); the LLG kernels' RK

@@ -18,7 +18,7 @@
 // read twice and stays in L2 between the launches for films up to ~2 M cells
 // in FP32.  Small films are bound by launch latency (three launches instead
 // of eight), large ones by the shared-memory passes and the barriers between
-// them (256x256x32 FP32: 38 + 43 + 28 us, where memory needs ~35 in all).
+// them (256x256x32 FP32: 43 + 50 + 33 us, where its 84 bytes per cell take 27).
 //
 // The transforms are Stockham autosort passes in shared memory, two buffers
 // used in turn, each butterfly in registers.  A pass spreads its butterflies

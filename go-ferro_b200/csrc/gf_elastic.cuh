@@ -194,7 +194,8 @@ __device__ inline void eigen_glb(const Params& P, const StageIOT<R>& io, long c,
 // eigenstrain), where each cell's strain takes the face's own gradient for
 // the normal component and for the shear components that involve it; it is
 // 0 on stress-free faces, except for the surface traction source.  Every
-// expression keeps the reference's operation order (rounding included).
+// expression keeps the reference's operation order; its roundings differ where
+// multiply-adds contract and divisions are products with a reciprocal.
 // ---------------------------------------------------------------------------
 
 // elastic constants of one material, staged in shared memory

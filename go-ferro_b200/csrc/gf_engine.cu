@@ -120,8 +120,8 @@ struct gf_engine {
     double* flexo_pge[6] = {};
     ETileMaps etm[2][4] = {};          // TMA maps of k_elastic_tile per step parity and stage
     unsigned* tma_err = nullptr;       // set by a timed-out TMA wait
-    int el_chunk = 1;                  // x-planes per block of k_elastic_tile
-    int el_nmat = 0;                   // materials staged by k_elastic_tile
+    int el_chunk = 1;                  // x-planes per block of the stress divergence
+    int el_nmat = 0;                   // materials staged by a block of it
     size_t el_smem = 0;                // its dynamic shared memory
     bool el_cubic = false;             // every material has the cubic stiffness pattern
     // the only class of the E edges, of four material cells
@@ -217,7 +217,7 @@ int gf_mixed_enqueue_stage(gf_engine* eng, int parity, int s);         // kernel
 int gf_mixed_elastic_setup(gf_engine* eng, int* per_sm);             // shared-memory opt-in, occupancy
 int gf_mixed_conv_attr(gf_engine* eng);                                 // shared-memory opt-in of the convolution kernels
 int gf_mixed_col_setup(gf_engine* eng);                                 // the same for k_elastic_col, and its tile
-int gf_mixed_time_tile(gf_engine* eng, int reps, float* ms);          // stage-1 elastic tile, mean ms per launch
+int gf_mixed_time_tile(gf_engine* eng, int reps, float* ms);          // stage-1 stress divergence, mean ms per launch
 int gf_mixed_adj_elastic(gf_engine* eng, int s, int rk, const StageIOT<float>& io);  // adjoint: FP32 stress divergence / RK of stage s
 int gf_mixed_batch_attr();                                              // shared-memory opt-in of the batch phase kernels
 int gf_mixed_batch_persistent_blocks(size_t smem, int* blocks);          // co-resident blocks of k_batch_persistent
@@ -1194,7 +1194,7 @@ int enqueue_stage(gf_engine* eng, int parity) {
     // Maxwell update reads the LLG increment (M-sourced current, spin
     // pumping), and the PEC kernel clears the step-start E that the TDGL
     // kernel reads at stage 1.  So the elastic chain runs on the engine
-    // stream and the LLG, TDGL and Maxwell kernels on three branch streams
+    // stream and the LLG, TDGL, E and H kernels on four branch streams
     // forked from it and joined before the static solves; the tiny boundary
     // kernels and the tails of the big ones then overlap other physics.
     // (per-kernel timing, gf_profile_steps, keeps one stream: each kernel is
@@ -1300,7 +1300,7 @@ int enqueue_stage(gf_engine* eng, int parity) {
     return GF_OK;
 }
 
-// Mean device time of `reps` launches of the stage-1 elastic tile kernel at
+// Mean device time of `reps` launches of the stage-1 stress divergence at
 // the engine's current x-chunk.  The kernel writes only per-stage scratch (the
 // stress divergence and the cell strain), so timing it leaves the state alone.
 template <class R>
@@ -2092,15 +2092,16 @@ int create_from(gf_engine* eng, const std::string& dir, int device, int precisio
     {
         // Priorities of the stage kernels' streams, kept by the step
         // graph's kernel nodes (cudaGraphInstantiateFlagUseNodePriority).
-        // Without magnets the elastic chain of the engine stream (tile, RK
-        // update) is the longest of a stage and goes first, then the
-        // Maxwell update and the TDGL kernel in the order measured faster
+        // Without magnets the elastic chain of the engine stream (stress
+        // divergence, RK update) is the longest of a stage and goes first, then
+        // the Maxwell update and the TDGL kernel in the order measured faster
         // for each form (128^3 ferroelectric, ms per step: FP64 1.513 with
-        // Maxwell before TDGL, 1.530 the other way; FP32 TDGL before Maxwell).  With magnets the
-        // LLG and Maxwell kernels wait for the tile and RK update is off the
-        // critical path: equal priorities (128x128x96 magnetoelastic: the
-        // elastic-first order measured 0.878 -> 0.905 ms FP32, 1.491 ->
-        // 1.521 FP64; branches first 0.880 / 1.492).
+        // Maxwell before TDGL, 1.530 the other way; FP32 TDGL before Maxwell).
+        // With magnets the LLG kernel, and the H faces after it, wait for the
+        // stress divergence and the RK update is off the critical path: equal
+        // priorities (128x128x96 magnetoelastic, measured with the general tile
+        // and one Yee kernel: the elastic-first order 0.878 -> 0.905 ms FP32,
+        // 1.491 -> 1.521 FP64; branches first 0.880 / 1.492).
         int lo = 0, hi = 0;
         GF_CU(cudaDeviceGetStreamPriorityRange(&lo, &hi));
         const int mid = (lo + hi) / 2;
@@ -2250,7 +2251,7 @@ int create_from(gf_engine* eng, const std::string& dir, int device, int precisio
     }
     if (d.elastodynamics)
         for (int a = 0; a < 9; a++) GF_TRY(dalloc_r(eng, &eng->fg[a], (size_t)n));
-    // the crystal-frame cell strain the elastic tile hands to the LLG kernels
+    // the crystal-frame cell strain the elastic kernel hands to the LLG kernels
     if (d.elastodynamics && P.elasto_on && (P.fm || P.afm))
         for (int a = 0; a < 6; a++) GF_TRY(dalloc_r(eng, &eng->strain_c[a], (size_t)n));
     // flexoelectricity: global-frame cell strain and eigenstrain p-gradients
@@ -4581,7 +4582,7 @@ cudaError_t adj_eval_launch(gf_adjoint* a, F3T<R> y, F3T<R> hd, V3<R> he, F3T<R>
 // the stage states to Y (m) and US / VS (u, v), the stage strains to STR;
 // stage 4 writes m to xout (compensation words to xcout in FP32; x itself in
 // the forward run) and leaves the new u, v in UACC / VACC.  The elastic
-// parts run the engine's own k_elastic_tile and k_elastic_rk (so the forward
+// parts run the engine's own k_elastic_col and k_elastic_rk (so the forward
 // run is the engine's discretisation); k_elastic_rk of stage 1 stores the
 // step's stage-1 force in x's fs.
 template <class R>

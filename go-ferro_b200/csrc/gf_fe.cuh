@@ -24,7 +24,7 @@ __device__ inline bool is_fe(const DevMatT<R>* mats, uint8_t id) {
 // 106-227), formed from u_in directly: the face-normal gradient on each of
 // the six faces (0 on stress-free faces: a non-periodic end face, or vacuum
 // on either side), averaged per component exactly as the stored face
-// gradients are in k_elastic_tile.  u = the cell's displacement, un = the
+// gradients are in the elastic kernels.  u = the cell's displacement, un = the
 // six neighbours' (-x, +x, -y, +y, -z, +z, wrapped), solid_nb = whether each
 // neighbour is a material cell.  gn, when given, receives the normal
 // gradients gn[d][0 / 1] = d u_d / d x_d on the -d / +d face.

@@ -33,7 +33,7 @@ __device__ inline bool is_fm(const DevMat* mats, uint8_t id) {
 
 // static strain plus the cell strain of the stage displacement, crystal
 // frame (exxt0_crt + Dexx_crt, magnetic_solver.cpp:89-96); the dynamic part
-// is written by k_elastic_tile earlier in the same stage
+// is written by the elastic kernel earlier in the same stage
 template <class R>
 __device__ inline void cell_strain_total(const Params& P, const StageIOT<R>& io, long i, long j, long k, long c, R e[6]) {
     R d[6] = {R(0), R(0), R(0), R(0), R(0), R(0)};

@@ -121,16 +121,20 @@ typedef struct gf_kernel_time {
 int gf_create_from_deck(const char* deck_dir, int device, gf_engine** out);
 
 /* Arithmetic of an engine (gf_create_from_deck_ex).
- *   GF_PRECISION_FP64: every field, stencil and transform in FP64, evaluated
- *     in the reference's operation order (the parity form).
+ *   GF_PRECISION_FP64: every field, stencil and transform in FP64 (the parity
+ *     form).  The formulas are the reference's, not its roundings: the kernels
+ *     contract multiply-adds, multiply by rounded reciprocals of the cell
+ *     sizes, dt and most RK weights, and the elastic stress of cubic decks is
+ *     summed cell by cell.  A step agrees with the reference to about 1e-15 per
+ *     term.
  *   GF_PRECISION_MIXED_FP32: state arrays, stencils and FFTs in FP32; each
  *     state scalar carries an FP32 compensation word, so the RK4 step value
  *     X + C accumulates increments without FP32 rounding drift; |m| is
  *     renormalised to 1 after every stage (the reference does not
  *     renormalise).  The demag tensor and its spectra are built in FP64; the
  *     averages and every upload/download stay FP64 at this ABI.
- *     Every physics of the FP64 form runs in both; the electrostatic
- *     solve and the adjoint are FP64 only. */
+ *     Every physics of the FP64 form runs in both; the spectral
+ *     electrostatic solve is FP64 only. */
 #define GF_PRECISION_FP64 0
 #define GF_PRECISION_MIXED_FP32 1
 
@@ -556,14 +560,16 @@ void gf_adjoint_destroy(gf_adjoint* a);
  * Errors are reported through gf_last_error(NULL). */
 int gf_field_mean_noalloc(const double* dev_in, uint64_t n, double divisor, double* dev_out, void* stream);
 
-/* Diagnostic: the stencil kernels divide by run constants (cell sizes, dt,
- * the RK4 weights 3 and 6) with a reciprocal-and-correction sequence
- * instead of the general division.  This queues, on the current device,
- * n quotients x / d for pseudo-random x of magnitude 1e-30..1e30 (half of
- * them close to rounding midpoints) with seed `seed`, computes each both
- * ways and stores in *mismatches how many differ in any bit.  No
- * counterpart in the reference; the reference divides with IEEE division,
- * so 0 mismatches means the kernels' quotients equal the reference's. */
+/* Diagnostic of the one exact division the FP64 kernels still form: the LLG
+ * kernels divide their RK4 increments by 3 and 6 with a
+ * reciprocal-and-correction sequence instead of the general division.  (The
+ * stencils and the other kernels multiply by the rounded reciprocal, within
+ * two ulps of the quotient; this call says nothing about those.)  It queues, on
+ * the current device, n quotients x / d for pseudo-random x of magnitude
+ * 1e-30..1e30 (half of them close to rounding midpoints) with seed `seed`,
+ * computes each both ways and stores in *mismatches how many differ in any
+ * bit.  No counterpart in the reference, which divides with IEEE division: 0
+ * mismatches for d = 3 and 6 means those quotients equal the reference's. */
 int gf_check_quotients(double d, uint64_t n, uint64_t seed, uint64_t* mismatches);
 
 /* Library version string. */

@@ -1,8 +1,10 @@
-"""The stencil kernels divide by run constants (cell sizes, dt, the RK4
-weights 3 and 6) with a precomputed reciprocal and two residual corrections
-instead of the general division.  The reference divides with IEEE division;
-these tests check, through gf_check_quotients, that both give the same bits
-on many numerators, half of them chosen next to rounding midpoints."""
+"""The LLG kernels divide by the RK4 weights 3 and 6 with a precomputed
+reciprocal and two residual corrections instead of the general division.  The
+reference divides with IEEE division; these tests check, through
+gf_check_quotients, that both give the same bits on many numerators, half of
+them chosen next to rounding midpoints.  The sequence holds for any divisor, so
+others are tried too; the stencils do not use it (they multiply by the rounded
+reciprocal of the cell sizes and dt), and nothing here covers them."""
 import ctypes
 import math
 
