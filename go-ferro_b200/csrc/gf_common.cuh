@@ -81,6 +81,7 @@ struct Params {
     long n;
     double dx, dy, dz, dt;
     double rdx, rdy, rdz, rdt;   // correctly rounded reciprocals (host 1./dx ...), for qdivR
+    double rdxl, rdyl, rdzl;     // 1/dx - rdx ..., rounded, for qdiv2
     double dt_e0, mdt_mu0;       // dt / e0 and -dt / mu0, rounded as the reference does
     int rot;                 // if_OrientRotate
     double Tg2c[3][3], Tc2g[3][3];
@@ -149,8 +150,17 @@ struct StepDrive {
     StageDrive st[4];
 };
 
+// a product rounded by itself (never contracted) and a fused multiply-add
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+
 constexpr double kInv3 = 1. / 3.;
 constexpr double kInv6 = 1. / 6.;
+// 1/3 - kInv3 and 1/6 - kInv6, rounded, for qdiv2
+constexpr double kInv3l = 0x1.5555555555555p-56;
+constexpr double kInv6l = 0x1.5555555555555p-57;
 
 // x / d rounded to nearest, for a divisor d that is fixed for the run, given
 // rd = RN(1/d) (computed once on the host by IEEE division).  This is
@@ -172,6 +182,13 @@ __device__ __forceinline__ double qdiv(double x, double d, double rd) {
     const double q2 = __fma_rn(r, rd, q1);
     return x == 0. ? q0 : q2;
 }
+
+// x / d rounded to nearest but for numerators whose quotient lies within 2^-53
+// of its size from a rounding midpoint, given rd = RN(1/d) and rl = RN(1/d - rd)
+// (N. Brisebarre, J.-M. Muller and S. K. Raina, "Accelerating correctly rounded
+// floating-point division when the divisor is known in advance", IEEE Trans.
+// Comput. 53(8), 2004): two operations, for sums of quotients that nearly cancel.
+__device__ __forceinline__ double qdiv2(double x, double rd, double rl) { return __fma_rn(x, rd, __dmul_rn(x, rl)); }
 
 // Division by a run constant d in the stencils: a multiplication by its
 // rounded reciprocal (rd = RN(1/d), rdf in FP32): two roundings, within two ulps

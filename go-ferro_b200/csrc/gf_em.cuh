@@ -163,13 +163,29 @@ __device__ inline void edge_load(const Params& P, const StageIOT<R>& io, const E
     }
 }
 
+// a / da - b / db, the curl of a component (ra = RN(1/da), la its remainder).
+// The curl of a gradient (the field of charges) cancels: FP64 forms both
+// quotients as the division would round them, so that equal ones cancel exactly
+// and what is left carries the noise of the operands only.  A product contracted
+// into the difference leaves the rounding error of the other one instead (sheet
+// currents of a box, H along the current 1e-6 of the field: 2.8e-10 of that
+// component from the divisions' rounding, with the reference's quotients
+// 2.7e-11).  In FP32 the rounding of the fields is what shows.
+__device__ __forceinline__ float yee_diff(float a, float ra, float b, float rb, double, double) { return fma_rn(a, ra, -mul_rn(b, rb)); }
+__device__ __forceinline__ double yee_diff(double a, double ra, double b, double rb, double la, double lb) {
+    return qdiv2(a, ra, la) - qdiv2(b, rb, lb);
+}
+
 // curl from the gathered operands; component C's two grid spacings are
 // (y, z), (z, x), (x, y)
 template <int C, class R>
 __device__ inline R yee_curl(const Params& P, const YeeIn<R>& L) {
-    if (C == 0) return qdivR(L.c[0] - L.c[1], P.dy, P.rdy, P.f.rdy) - qdivR(L.c[2] - L.c[3], P.dz, P.rdz, P.f.rdz);
-    if (C == 1) return qdivR(L.c[0] - L.c[1], P.dz, P.rdz, P.f.rdz) - qdivR(L.c[2] - L.c[3], P.dx, P.rdx, P.f.rdx);
-    return qdivR(L.c[0] - L.c[1], P.dx, P.rdx, P.f.rdx) - qdivR(L.c[2] - L.c[3], P.dy, P.rdy, P.f.rdy);
+    R rx, ry, rz;
+    if constexpr (is_mixed<R>::value) { rx = P.f.rdx; ry = P.f.rdy; rz = P.f.rdz; }
+    else { rx = P.rdx; ry = P.rdy; rz = P.rdz; }
+    if (C == 0) return yee_diff(L.c[0] - L.c[1], ry, L.c[2] - L.c[3], rz, P.rdyl, P.rdzl);
+    if (C == 1) return yee_diff(L.c[0] - L.c[1], rz, L.c[2] - L.c[3], rx, P.rdzl, P.rdxl);
+    return yee_diff(L.c[0] - L.c[1], rx, L.c[2] - L.c[3], ry, P.rdxl, P.rdyl);
 }
 
 template <int S, class R>
@@ -186,10 +202,10 @@ __device__ inline void rk_x(const YeeIn<R>& L, R d, R* out, R* acc, R* cmp, int 
             cmp[e] = err;
         }
     } else {
-        if (S == 0) { out[e] = xv + d * 0.5; acc[e] = xv + d * kInv6; }
-        else if (S == 1) { out[e] = xv + d * 0.5; acc[e] = L.acc + d * kInv3; }
-        else if (S == 2) { out[e] = xv + d; acc[e] = L.acc + d * kInv3; }
-        else { acc[e] = L.acc + d * kInv6; }
+        if (S == 0) { out[e] = xv + d * 0.5; acc[e] = xv + qdiv2(d, kInv6, kInv6l); }
+        else if (S == 1) { out[e] = xv + d * 0.5; acc[e] = L.acc + qdiv2(d, kInv3, kInv3l); }
+        else if (S == 2) { out[e] = xv + d; acc[e] = L.acc + qdiv2(d, kInv3, kInv3l); }
+        else { acc[e] = L.acc + qdiv2(d, kInv6, kInv6l); }
     }
 }
 
@@ -429,8 +445,9 @@ __global__ void __launch_bounds__(256, is_mixed<R>::value ? GF_EM_MINB_F32 : GF_
 // what their curls and sources read (9 distinct H values where k_em_fused
 // loads 12 and re-derives the cells per edge), the three faces the vertex's E
 // (9 of 12), and material ids and dM/dt are read only with M sources.
-// Products that feed a sum are fma(), so that the batched kernels give the
-// same bits.
+// Products that feed a sum are fma() or rounded by themselves, so that the
+// batched kernels give the same bits; the quotients of the curls and of the RK
+// weights are yee_diff's and qdiv2's.
 // ---------------------------------------------------------------------------
 // NC: through the read-only path; a kernel that also writes the array between
 // grid barriers (the persistent batch step) reads it plainly
@@ -451,10 +468,10 @@ __device__ __forceinline__ void yee_rk(R x, R av, R cv, R d, R* out, R* acc, R* 
             cmp[e] = err;
         }
     } else {
-        if (S == 0) { out[e] = fma_rn(d, 0.5, x); acc[e] = fma_rn(d, kInv6, x); }
-        else if (S == 1) { out[e] = fma_rn(d, 0.5, x); acc[e] = fma_rn(d, kInv3, av); }
-        else if (S == 2) { out[e] = x + d; acc[e] = fma_rn(d, kInv3, av); }
-        else { acc[e] = fma_rn(d, kInv6, av); }
+        if (S == 0) { out[e] = fma_rn(d, 0.5, x); acc[e] = x + qdiv2(d, kInv6, kInv6l); }
+        else if (S == 1) { out[e] = fma_rn(d, 0.5, x); acc[e] = av + qdiv2(d, kInv3, kInv3l); }
+        else if (S == 2) { out[e] = x + d; acc[e] = av + qdiv2(d, kInv3, kInv3l); }
+        else { acc[e] = av + qdiv2(d, kInv6, kInv6l); }
     }
 }
 
@@ -515,8 +532,8 @@ __device__ __forceinline__ void yee_E_body(const Params& P, const StageIOT<R>& i
     }
     const bool yb = (j == 0 || j == ny) && !P.per_y, zb = (k == 0 || k == nz) && !P.per_z, xb = (i == 0 || i == nx) && !P.per_x;
     const bool bnd[3] = {yb || zb, xb || zb, xb || yb};
-    const R curl[3] = {fma_rn(hzb - hzj, ry, -mul_rn(hyb - hyk, rz)), fma_rn(hxb - hxk, rz, -mul_rn(hzb - hzi, rx)),
-                       fma_rn(hyb - hyi, rx, -mul_rn(hxb - hxj, ry))};
+    const R curl[3] = {yee_diff(hzb - hzj, ry, hyb - hyk, rz, P.rdyl, P.rdzl), yee_diff(hxb - hxk, rz, hzb - hzi, rx, P.rdzl, P.rdxl),
+                       yee_diff(hyb - hyi, rx, hxb - hxj, ry, P.rdxl, P.rdyl)};
     R jf[3] = {z, z, z};
     if (P.jf_on && ((km >= P.jf_k0 && km <= P.jf_k1) || (kw >= P.jf_k0 && kw <= P.jf_k1))) {
         const R a = R(stage_drive(io, S).jf);
@@ -539,7 +556,9 @@ __device__ __forceinline__ void yee_E_body(const Params& P, const StageIOT<R>& i
     for (int c = 0; c < 3; c++) {
         if (!on[c]) continue;
         const EmCls<R>& ec = UNI ? uc : cl[kc[c]];
-        R rhs = fma_rn(-ec.cond, self[c], curl[c] - jf[c]);
+        R rhs;
+        if constexpr (is_mixed<R>::value) rhs = fma_rn(-ec.cond, self[c], curl[c] - jf[c]);
+        else rhs = (curl[c] - jf[c]) - mul_rn(ec.cond, self[c]);
         if constexpr (FROMP) {
             const uint32_t mask = UNI ? 15u : ec.mask;
             R sum = z;
@@ -609,15 +628,20 @@ __device__ __forceinline__ void yee_H_body(const Params& P, const StageIOT<R>& i
             const R ma = sMs[ldro<NC>(io.mid + a)], mb = sMs[ldro<NC>(io.mid + b)];
             R sum = z;
             if (ma != z) sum = mul_rn(da, ma);
-            if (mb != z) sum = fma_rn(db, mb, sum);
+            if constexpr (is_mixed<R>::value) { if (mb != z) sum = fma_rn(db, mb, sum); }
+            else { if (mb != z) sum = sum + mul_rn(db, mb); }
             dms[c] = (ma != z && mb != z) ? mul_rn(sum, R(0.5)) : sum;
         }
     }
-    const R curl[3] = {fma_rn(n[0] - s2, ry, -mul_rn(n[1] - s1, rz)), fma_rn(n[2] - s0, rz, -mul_rn(n[3] - s2, rx)),
-                       fma_rn(n[4] - s1, rx, -mul_rn(n[5] - s0, ry))};
+    const R curl[3] = {yee_diff(n[0] - s2, ry, n[1] - s1, rz, P.rdyl, P.rdzl), yee_diff(n[2] - s0, rz, n[3] - s2, rx, P.rdzl, P.rdxl),
+                       yee_diff(n[4] - s1, rx, n[5] - s0, ry, P.rdxl, P.rdyl)};
 #pragma unroll
     for (int c = 0; c < 3; c++)
-        if (on[c]) yee_rk<S>(x[c], av[c], cv[c], fma_rn(mdt, curl[c], -dms[c]), io.H_out.c[c], io.H_acc.c[c], io.H_cmp.c[c], e[c]);
+        if (on[c]) {
+            R d;
+            if constexpr (is_mixed<R>::value) d = fma_rn(mdt, curl[c], -dms[c]); else d = mul_rn(mdt, curl[c]) - dms[c];
+            yee_rk<S>(x[c], av[c], cv[c], d, io.H_out.c[c], io.H_acc.c[c], io.H_cmp.c[c], e[c]);
+        }
 }
 
 // Blocks of 256 threads per SM the registers allow: as many as keep a thread's

@@ -468,6 +468,7 @@ void build_params(gf_engine* eng) {
     P.per_x = d.per_x; P.per_y = d.per_y; P.per_z = d.per_z;
     P.dx = d.dx; P.dy = d.dy; P.dz = d.dz; P.dt = d.dt;
     P.rdx = 1. / d.dx; P.rdy = 1. / d.dy; P.rdz = 1. / d.dz; P.rdt = 1. / d.dt;
+    P.rdxl = std::fma(-P.rdx, d.dx, 1.) / d.dx; P.rdyl = std::fma(-P.rdy, d.dy, 1.) / d.dy; P.rdzl = std::fma(-P.rdz, d.dz, 1.) / d.dz;
     P.dt_e0 = d.dt / kE0; P.mdt_mu0 = -d.dt / kMu0;
     P.rot = d.orient_rotate;
     for (int i = 0; i < 3; i++) for (int j = 0; j < 3; j++) { P.Tg2c[i][j] = d.Tg2c[i][j]; P.Tc2g[i][j] = d.Tc2g[i][j]; }

@@ -216,6 +216,30 @@ def test_yee_update_equals_the_general_one(gf, name, precision):
     _same(_run(gf, d, precision), _run(gf, g, precision), TOL[precision])
 
 
+# Differences that are zero before any rounding, so every term of them has to be
+# formed such that equal ones cancel exactly: 0 and no other value.
+@pytest.mark.parametrize("general", [False, True])
+def test_curl_of_a_gradient_is_zero(gf, general):
+    """E = grad(3 y z): dE_z/dy = dE_y/dz in every cell, so no H grows (FP64)."""
+    nx, ny, nz = 4, 24, 24
+    d = _fe(gf, nx, ny, nz, elastic=False, elasto_back=False, elasto_on=False, em_fromP=False, em_back_P=False, jf=False,
+            materials=[gf.decks.ggg()])
+    if general:
+        pole = dataclasses.replace(gf.decks.ggg(), drude=((1.0, 1e15, 1e-14), (0.0, 0.0, 1.0), (0.0, 0.0, 1.0)))
+        d.materials = d.materials + [pole]
+    d.p0 = d.q0 = None
+    with gf.Engine.from_params(d, device=0) as e:
+        Ey, Ez = e.download("Ey"), e.download("Ez")
+        Ey[:] = 3.0 * np.arange(nz + 1)
+        Ez[:] = 3.0 * np.arange(ny + 1)[:, None]
+        e.upload("Ey", Ey)
+        e.upload("Ez", Ez)
+        e.advance(1)
+        # the ramps break at the ends, one cell further in per stage
+        for f in ("Hx", "Hy", "Hz"):
+            assert not np.any(e.download(f)[:, 6:-6, 6:-6]), f
+
+
 # sides with the transforms' radices 8, 4, 2, 3, 5 and their products, odd
 # ones, a single plane, row or layer, (49, 22, 250) three that cuFFT keeps, and
 # one whose x blocks take 8 columns with a remainder
