@@ -52,7 +52,7 @@ using C6 = C6T<double>;
 template <class R> struct V3 { R x, y, z; };
 template <class R> __host__ __device__ inline V3<R> mk3(R a, R b, R c) { return V3<R>{a, b, c}; }
 template <class R> __device__ inline V3<R> cross3(V3<R> a, V3<R> b) {
-    return mk3<R>(a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x);
+    return mk3<R>(cross_term(a.y, b.z, a.z, b.y), cross_term(a.z, b.x, a.x, b.z), cross_term(a.x, b.y, a.y, b.x));
 }
 template <class R> __device__ inline R dot3(V3<R> a, V3<R> b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
 template <class R> __device__ inline V3<R> ld3(const F3T<R>& f, int c) { return mk3<R>(f.c[0][c], f.c[1][c], f.c[2][c]); }

@@ -156,6 +156,16 @@ __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, 
 __device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
 __device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 
+// Ms1 m1 + Ms2 m2 of two sublattices, from rounded products: opposite ones
+// cancel exactly, where a contraction leaves the rounding error of one
+template <class R>
+__device__ __forceinline__ R moment_sum(R Ms1, R m1, R Ms2, R m2) { return mul_rn(Ms1, m1) + mul_rn(Ms2, m2); }
+// a b - c d of a cross product.  FP64 likewise: the torque on a moment along its
+// field is zero.  FP32 leaves the contraction to the compiler: its fields are
+// rounded far more coarsely.
+__device__ __forceinline__ double cross_term(double a, double b, double c, double d) { return mul_rn(a, b) - mul_rn(c, d); }
+__device__ __forceinline__ float cross_term(float a, float b, float c, float d) { return a * b - c * d; }
+
 constexpr double kInv3 = 1. / 3.;
 constexpr double kInv6 = 1. / 6.;
 // 1/3 - kInv3 and 1/6 - kInv6, rounded, for qdiv2

@@ -201,12 +201,12 @@ static __global__ void k_mag_source(Params P, const DevMat* mats, const uint8_t*
     } else if (fl & MF_AFM) {
         const double Ms1 = mats[id - 1].Ms1, Ms2 = mats[id - 1].Ms2;
         if (mode == 0) {
-            for (int a = 0; a < 3; a++) M3[a * P.n + c] = Ms1 * a1.c[a][c] + Ms2 * a2.c[a][c];
+            for (int a = 0; a < 3; a++) M3[a * P.n + c] = moment_sum(Ms1, a1.c[a][c], Ms2, a2.c[a][c]);
         } else if (mode == 1) {
             const double f[3] = {f0, f1, f2};
-            for (int a = 0; a < 3; a++) Hs.c[a][c] = (Ms1 * a1.c[a][c] + Ms2 * a2.c[a][c]) * f[a];
+            for (int a = 0; a < 3; a++) Hs.c[a][c] = moment_sum(Ms1, a1.c[a][c], Ms2, a2.c[a][c]) * f[a];
         } else {
-            Hs.c[0][c] = 0.; Hs.c[1][c] = 0.; Hs.c[2][c] = -Ms1 * a1.c[2][c] - Ms2 * a2.c[2][c];
+            Hs.c[0][c] = 0.; Hs.c[1][c] = 0.; Hs.c[2][c] = -moment_sum(Ms1, a1.c[2][c], Ms2, a2.c[2][c]);
         }
     } else if (mode == 0) {
         M3[c] = 0.; M3[P.n + c] = 0.; M3[2 * P.n + c] = 0.;
@@ -252,12 +252,12 @@ static __global__ void k_mag_source_f32(Params P, const DevMatT<float>* mats, co
     } else if (fl & MF_AFM) {
         const float Ms1 = mats[id - 1].Ms1, Ms2 = mats[id - 1].Ms2;
         if (mode == 0) {
-            for (int a = 0; a < 3; a++) M3[a * P.n + c] = Ms1 * a1.c[a][c] + Ms2 * a2.c[a][c];
+            for (int a = 0; a < 3; a++) M3[a * P.n + c] = moment_sum(Ms1, a1.c[a][c], Ms2, a2.c[a][c]);
         } else if (mode == 1) {
             const float f[3] = {f0, f1, f2};
-            for (int a = 0; a < 3; a++) Hs.c[a][c] = (Ms1 * a1.c[a][c] + Ms2 * a2.c[a][c]) * f[a];
+            for (int a = 0; a < 3; a++) Hs.c[a][c] = moment_sum(Ms1, a1.c[a][c], Ms2, a2.c[a][c]) * f[a];
         } else {
-            Hs.c[0][c] = 0.f; Hs.c[1][c] = 0.f; Hs.c[2][c] = -Ms1 * a1.c[2][c] - Ms2 * a2.c[2][c];
+            Hs.c[0][c] = 0.f; Hs.c[1][c] = 0.f; Hs.c[2][c] = -moment_sum(Ms1, a1.c[2][c], Ms2, a2.c[2][c]);
         }
     } else if (mode == 0) {
         M3[c] = 0.f; M3[P.n + c] = 0.f; M3[2 * P.n + c] = 0.f;

@@ -71,10 +71,10 @@ __device__ inline R ishe_cell(const Params& P, const StageIOT<R>& io, int C, int
     if (sz < 0) return R(0.);
     const int s = (ci * P.ny + cj) * P.nz + sz;
     R sum = R(0.);
-    if (P.fm) sum = io.m_in.c[C][s] * io.dm.c[2][s] - io.m_in.c[2][s] * io.dm.c[C][s];
+    if (P.fm) sum = cross_term(io.m_in.c[C][s], io.dm.c[2][s], io.m_in.c[2][s], io.dm.c[C][s]);
     if (P.afm) {
-        sum = sum + io.a1_in.c[C][s] * io.da1.c[2][s] - io.a1_in.c[2][s] * io.da1.c[C][s];
-        sum = sum + io.a2_in.c[C][s] * io.da2.c[2][s] - io.a2_in.c[2][s] * io.da2.c[C][s];
+        sum = sum + cross_term(io.a1_in.c[C][s], io.da1.c[2][s], io.a1_in.c[2][s], io.da1.c[C][s]);
+        sum = sum + cross_term(io.a2_in.c[C][s], io.da2.c[2][s], io.a2_in.c[2][s], io.da2.c[C][s]);
     }
     return qdivR(io.ishe_coef[ck] * sum, P.dt, P.rdt, P.f.rdt);
 }
@@ -343,7 +343,7 @@ __device__ inline void em_H_face(const Params& P, const StageIOT<R>& io, const E
         const EmMat<R>& m = mt[L.t1 - 1];
         if (P.em_fromM) {
             dM1 = L.dm1 * m.Ms;
-            if (P.afm) dM1 = dM1 + io.da1.c[C][L.c1] * m.Ms1 + io.da2.c[C][L.c1] * m.Ms2;
+            if (P.afm) dM1 = dM1 + moment_sum(m.Ms1, io.da1.c[C][L.c1], m.Ms2, io.da2.c[C][L.c1]);
         }
         if (m.flags & (MF_FM | MF_AFM)) cnt = cnt + R(1.);
     }
@@ -351,7 +351,7 @@ __device__ inline void em_H_face(const Params& P, const StageIOT<R>& io, const E
         const EmMat<R>& m = mt[L.t2 - 1];
         if (P.em_fromM) {
             dM2 = L.dm2 * m.Ms;
-            if (P.afm) dM2 = dM2 + io.da1.c[C][L.c2] * m.Ms1 + io.da2.c[C][L.c2] * m.Ms2;
+            if (P.afm) dM2 = dM2 + moment_sum(m.Ms1, io.da1.c[C][L.c2], m.Ms2, io.da2.c[C][L.c2]);
         }
         if (m.flags & (MF_FM | MF_AFM)) cnt = cnt + R(1.);
     }

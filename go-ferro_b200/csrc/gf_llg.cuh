@@ -227,17 +227,17 @@ __global__ void __launch_bounds__(256, is_mixed<R>::value ? GF_LLG_MINB_F32 : GF
             // with the 1-D magnetostatic model the cell's Maxwell H_z is
             // -Ms m_z - H_stat,z of the stage state (:3793-3804; the
             // sublattice terms are zero in a ferromagnetic cell)
-            if (P.mag1d_em) Hz = Hz + (-R(1.) * mat.Ms * mzc - hs[2]);
+            if (P.mag1d_em) Hz = Hz + (-mul_rn(mat.Ms, mzc) - hs[2]);
             else Hz = Hz + (io.H_in.c[2][hz0] + io.H_in.c[2][hz1]) / R(2.);
         }
 
         const R precess = mat.precess;
-        const R px = myc * Hz - mzc * Hy;
-        const R py = mzc * Hx - mxc * Hz;
-        const R pz = mxc * Hy - myc * Hx;
-        const R qx = myc * pz - mzc * py;
-        const R qy = mzc * px - mxc * pz;
-        const R qz = mxc * py - myc * px;
+        const R px = cross_term(myc, Hz, mzc, Hy);
+        const R py = cross_term(mzc, Hx, mxc, Hz);
+        const R pz = cross_term(mxc, Hy, myc, Hx);
+        const R qx = cross_term(myc, pz, mzc, py);
+        const R qy = cross_term(mzc, px, mxc, pz);
+        const R qz = cross_term(mxc, py, myc, px);
         dmx = precess * px + mat.alpha_precess * qx;
         dmy = precess * py + mat.alpha_precess * qy;
         dmz = precess * pz + mat.alpha_precess * qz;
@@ -387,8 +387,7 @@ __global__ void __launch_bounds__(256, 2) k_llg_afm(Params P, StageIOT<R> io, co
                 // the 1-D model's H_z of the stage state (:3793-3804)
                 const DevMatT<R>& dm_ = io.mats[id - 1];
                 const R mzc = P.fm ? io.m_in.c[2][c] : R(0.);
-                Hem[2] = -R(1.) * dm_.Ms * mzc - R(1.) * dm_.Ms1 * io.a1_in.c[2][c] - R(1.) * dm_.Ms2 * io.a2_in.c[2][c]
-                         - io.Hstat.c[2][c];
+                Hem[2] = -(mul_rn(dm_.Ms, mzc) + moment_sum(dm_.Ms1, io.a1_in.c[2][c], dm_.Ms2, io.a2_in.c[2][c])) - io.Hstat.c[2][c];
             } else {
                 Hem[2] = (io.H_in.c[2][hz0] + io.H_in.c[2][hz1]) / R(2.);
             }
@@ -447,12 +446,12 @@ __global__ void __launch_bounds__(256, 2) k_llg_afm(Params P, StageIOT<R> io, co
             R Hy = io.Hstat.c[1][c] + Hay + Hmy + Hex[1] + Hiy + R(dr.Hext_afm[1]);
             R Hz = io.Hstat.c[2][c] + Haz + Hmz + Hex[2] + Hiz + R(dr.Hext_afm[2]);
             if (P.em_back_M) { Hx = Hx + Hem[0]; Hy = Hy + Hem[1]; Hz = Hz + Hem[2]; }
-            const R px = mgy * Hz - mgz * Hy;
-            const R py = mgz * Hx - mgx * Hz;
-            const R pz = mgx * Hy - mgy * Hx;
-            const R qx = mgy * pz - mgz * py;
-            const R qy = mgz * px - mgx * pz;
-            const R qz = mgx * py - mgy * px;
+            const R px = cross_term(mgy, Hz, mgz, Hy);
+            const R py = cross_term(mgz, Hx, mgx, Hz);
+            const R pz = cross_term(mgx, Hy, mgy, Hx);
+            const R qx = cross_term(mgy, pz, mgz, py);
+            const R qy = cross_term(mgz, px, mgx, pz);
+            const R qz = cross_term(mgx, py, mgy, px);
             dm[s][0] = mat.prec[s] * px + mat.aprec[s] * qx;
             dm[s][1] = mat.prec[s] * py + mat.aprec[s] * qy;
             dm[s][2] = mat.prec[s] * pz + mat.aprec[s] * qz;
@@ -561,7 +560,7 @@ __global__ void k_em_cell_hz_1d(const DevMatT<R>* __restrict__ mats, const uint8
     if (id == 0) { out[c] = 0.; return; }
     const DevMatT<R>& m = mats[id - 1];
     const R z = mz ? mz[c] : R(0.), z1 = mz1 ? mz1[c] : R(0.), z2 = mz2 ? mz2[c] : R(0.);
-    out[c] = (double)(-R(1.) * m.Ms * z - R(1.) * m.Ms1 * z1 - R(1.) * m.Ms2 * z2 - hz[c]);
+    out[c] = (double)(-(mul_rn(m.Ms, z) + moment_sum(m.Ms1, z1, m.Ms2, z2)) - hz[c]);
 }
 
 }  // namespace gf

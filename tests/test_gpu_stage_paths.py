@@ -240,6 +240,31 @@ def test_curl_of_a_gradient_is_zero(gf, general):
             assert not np.any(e.download(f)[:, 6:-6, 6:-6]), f
 
 
+def test_opposite_sublattices_have_no_moment(gf):
+    D = gf.decks
+    d = D.preset_fm_demag(nx=6, ny=5, nz=4, steps=5)
+    d.materials, d.m0, d.Hext_table = [D.afm_uniaxial(0.02)], None, None
+    m = _unit(np.random.default_rng(59), (6, 5, 4))
+    d.afm0 = np.concatenate([m, -m])
+    for kw in ({}, {"mag_1D": True}, {"demag_factor": True, "demag_fac": (0.1, 0.2, 0.7)}):
+        for precision in ("fp64", "mixed"):
+            with gf.Engine.from_params(dataclasses.replace(d, **kw), device=0, precision=precision) as e:
+                assert not np.any(e.download("Hstat")), (kw, precision)
+
+
+def test_a_moment_along_its_field_stays(gf):
+    """m and H along the diagonal of the film plane (FP64): no torque."""
+    D = gf.decks
+    d = D.preset_fm_demag(nx=4, ny=6, nz=3, steps=5)
+    d.magnetostatics, d.Hext_table, d.Hext_stat = False, None, (81234.5, 81234.5, 0.0)
+    d.materials = [dataclasses.replace(D.yig(0.02), K1=0.0)]
+    d.m0 = np.zeros((3, 4, 6, 3))
+    d.m0[:2] = np.sqrt(0.5)
+    with gf.Engine.from_params(d, device=0) as e:
+        e.advance(3)
+        assert np.array_equal(e.download("m"), d.m0)
+
+
 # sides with the transforms' radices 8, 4, 2, 3, 5 and their products, odd
 # ones, a single plane, row or layer, (49, 22, 250) three that cuFFT keeps, and
 # one whose x blocks take 8 columns with a remainder
