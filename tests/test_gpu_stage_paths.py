@@ -240,6 +240,25 @@ def test_curl_of_a_gradient_is_zero(gf, general):
             assert not np.any(e.download(f)[:, 6:-6, 6:-6]), f
 
 
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("layers", [[(12, 1)], [(4, 2), (6, 1), (2, 0)]])
+@pytest.mark.parametrize("rotated", [False, True])
+def test_laterally_uniform_stress_has_no_lateral_force(gf, layers, rotated, precision):
+    D = gf.decks
+    d = _fe(gf, 5, 14, 12, em=False, em_fromP=False, em_back_P=False, jf=False, materials=[D.pto(), D.ggg()], layers=layers)
+    if rotated:
+        d = dataclasses.replace(d, Tg2c=np.eye(3))     # the general tile
+    # a polarisation whose shear eigenstrains vanish and normal ones do not
+    d.p0 = np.zeros((3, 5, 14, 12))
+    d.p0[2] = 0.31 * (d.material_cell() == 1)
+    d.q0 = np.zeros_like(d.p0)
+    with gf.Engine.from_params(d, device=0, precision=precision) as e:
+        e.advance(3)
+        f, u = e.download("force_store"), e.download("u")
+    assert np.any(f[2])
+    assert not np.any(f[:2]) and not np.any(u[:2])
+
+
 def test_opposite_sublattices_have_no_moment(gf):
     D = gf.decks
     d = D.preset_fm_demag(nx=6, ny=5, nz=4, steps=5)
