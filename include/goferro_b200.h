@@ -122,11 +122,12 @@ int gf_create_from_deck(const char* deck_dir, int device, gf_engine** out);
 
 /* Arithmetic of an engine (gf_create_from_deck_ex).
  *   GF_PRECISION_FP64: every field, stencil and transform in FP64 (the parity
- *     form).  The formulas are the reference's, not its roundings: the kernels
- *     contract multiply-adds, multiply by rounded reciprocals of the cell
- *     sizes, dt and most RK weights, and the elastic stress of cubic decks is
- *     summed cell by cell.  A step agrees with the reference to about 1e-15 per
- *     term.
+ *     form).  The formulas are the reference's, not every rounding of it: the
+ *     kernels contract multiply-adds, most divisions by run constants are
+ *     products with rounded reciprocals, and the elastic stress of cubic decks
+ *     is summed cell by cell.  What cancels in the reference (curls, cross
+ *     products, opposite sublattices, face stresses) cancels here too.  A step
+ *     agrees with the reference to about 1e-15 per term.
  *   GF_PRECISION_MIXED_FP32: state arrays, stencils and FFTs in FP32; each
  *     state scalar carries an FP32 compensation word, so the RK4 step value
  *     X + C accumulates increments without FP32 rounding drift; |m| is
@@ -563,8 +564,9 @@ int gf_field_mean_noalloc(const double* dev_in, uint64_t n, double divisor, doub
 /* Diagnostic of the one exact division the FP64 kernels still form: the LLG
  * kernels divide their RK4 increments by 3 and 6 with a
  * reciprocal-and-correction sequence instead of the general division.  (The
- * stencils and the other kernels multiply by the rounded reciprocal, within
- * two ulps of the quotient; this call says nothing about those.)  It queues, on
+ * Maxwell update's quotients take two operations and are correctly rounded but
+ * in rare cases; the other kernels multiply by the rounded reciprocal, within
+ * two ulps of the quotient.  This call says nothing about those.)  It queues, on
  * the current device, n quotients x / d for pseudo-random x of magnitude
  * 1e-30..1e30 (half of them close to rounding midpoints) with seed `seed`,
  * computes each both ways and stores in *mismatches how many differ in any
