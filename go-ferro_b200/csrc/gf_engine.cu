@@ -1251,9 +1251,10 @@ int enqueue_stage(gf_engine* eng, int parity) {
     GF_CU(rec(ev_tile, st));
     if (mag) {
         GF_CU(wait_(s_llg, ev_tile, 0));
-        if (P.fm) GF_CU(klaunch<true>(eng, "k_llg_fm", k_llg_fm<S, R>, dim3(blocks_for(P.fm_bj * P.fm_bk, kThreads), (unsigned)P.fm_bi),
+        // (a material that no cell has leaves an empty box)
+        if (P.fm && P.fm_bi > 0) GF_CU(klaunch<true>(eng, "k_llg_fm", k_llg_fm<S, R>, dim3(blocks_for(P.fm_bj * P.fm_bk, kThreads), (unsigned)P.fm_bi),
                                       dim3(kThreads), 0, s_llg, P, io, llg_tables<R>(eng), (int)eng->deck.mats.size()));
-        if (P.afm) GF_CU(klaunch<true>(eng, "k_llg_afm", k_llg_afm<S, R>, dim3(blocks_for(P.afm_bj * P.afm_bk, kThreads), (unsigned)P.afm_bi),
+        if (P.afm && P.afm_bi > 0) GF_CU(klaunch<true>(eng, "k_llg_afm", k_llg_afm<S, R>, dim3(blocks_for(P.afm_bj * P.afm_bk, kThreads), (unsigned)P.afm_bi),
                                        dim3(kThreads), 0, s_llg, P, io, llg_tables<R>(eng), (int)eng->deck.mats.size()));
         if (P.prescribed_m)
             GF_CU(klaunch(eng, "k_prescribed_m", k_prescribed_m<S, R>, dim3(blocks_for((long)P.nx * P.ny, kThreads)), dim3(kThreads), 0,
@@ -2320,8 +2321,13 @@ int ensure_graphs(gf_engine* eng) {
         int rc = enqueue_step(eng, par);
         cudaGraph_t g = nullptr;
         cudaError_t ce = cudaStreamEndCapture(eng->stream, &g);
-        if (rc != GF_OK) { if (g) cudaGraphDestroy(g); return rc; }
-        if (ce != cudaSuccess) { eng->err = std::string("stream capture: ") + cudaGetErrorString(ce); return GF_ECUDA; }
+        if (rc != GF_OK || ce != cudaSuccess) {
+            // the next call's own launch check must not see this failure
+            (void)cudaGetLastError();
+            if (g) cudaGraphDestroy(g);
+            if (rc == GF_OK) eng->err = std::string("stream capture: ") + cudaGetErrorString(ce);
+            return rc != GF_OK ? rc : GF_ECUDA;
+        }
         eng->graph[par] = g;
         GF_CU(cudaGraphInstantiate(&eng->gexec[par], g, eng->prio_nodes ? cudaGraphInstantiateFlagUseNodePriority : 0));
     }
@@ -3990,6 +3996,7 @@ int batch_capture(gf_batch* b, bool phases, cudaGraph_t* gout, cudaGraphExec_t* 
             cudaGraph_t g = nullptr;
             const cudaError_t ce = cudaStreamEndCapture(b->stream, &g);
             if (rc != GF_OK || ce != cudaSuccess) {
+                (void)cudaGetLastError();
                 if (g) cudaGraphDestroy(g);
                 if (rc == GF_OK) b->err = std::string("batch capture: ") + cudaGetErrorString(ce);
                 return rc != GF_OK ? rc : GF_ECUDA;
@@ -4016,6 +4023,7 @@ int batch_capture(gf_batch* b, bool phases, cudaGraph_t* gout, cudaGraphExec_t* 
         cudaGraph_t g = nullptr;
         cudaError_t ce2 = cudaStreamEndCapture(b->stream, &g);
         if (rc != GF_OK || ce != cudaSuccess || ce2 != cudaSuccess) {
+            (void)cudaGetLastError();
             if (g) cudaGraphDestroy(g);
             if (rc == GF_OK) b->err = std::string("batch capture: ") + cudaGetErrorString(ce != cudaSuccess ? ce : ce2);
             return rc != GF_OK ? rc : GF_ECUDA;

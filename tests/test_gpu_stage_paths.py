@@ -259,6 +259,17 @@ def test_laterally_uniform_stress_has_no_lateral_force(gf, layers, rotated, prec
     assert not np.any(f[:2]) and not np.any(u[:2])
 
 
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_magnetic_materials_that_no_cell_has(gf, precision):
+    """They change nothing (their kernels' boxes are empty)."""
+    D = gf.decks
+    d = _moving(_fe(gf, 6, 12, 10), 61)
+    want = _run(gf, d, precision)
+    got = _run(gf, dataclasses.replace(d, materials=d.materials + [D.yig(0.02), D.afm_uniaxial(0.01)]), precision)
+    assert not np.any(got.pop("m")) and not np.any(got.pop("m_afm1"))
+    _same(got, want, TOL[precision])
+
+
 def test_opposite_sublattices_have_no_moment(gf):
     D = gf.decks
     d = D.preset_fm_demag(nx=6, ny=5, nz=4, steps=5)
