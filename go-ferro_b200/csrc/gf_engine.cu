@@ -1193,8 +1193,9 @@ int enqueue_stage(gf_engine* eng, int parity) {
     // dependencies: the LLG kernels read the cell strain the elastic kernel
     // writes, flexoelectric runs read k_flexo_prep's arrays, the
     // Maxwell update reads the LLG increment (M-sourced current, spin
-    // pumping), and the PEC kernel clears the step-start E that the TDGL
-    // kernel reads at stage 1.  So the elastic chain runs on the engine
+    // pumping), the PEC kernel clears the step-start E that the TDGL
+    // kernel reads at stage 1, and the Liao boundary rewrites a plane of the
+    // step-start u that it reads then.  So the elastic chain runs on the engine
     // stream and the LLG, TDGL, E and H kernels on four branch streams
     // forked from it and joined before the static solves; the tiny boundary
     // kernels and the tails of the big ones then overlap other physics.
@@ -1273,6 +1274,11 @@ int enqueue_stage(gf_engine* eng, int parity) {
         GF_CU(rec(ev_emh, s_emh));
     }
     if (P.elastic) {
+        // The Liao boundary of stage 1 rewrites the k = 0 plane of the step value,
+        // which is that stage's input of the TDGL kernel (its strain).  The plane
+        // changes only where it is not the boundary's own last value: after a
+        // restart or an upload of u.
+        if (S == 0 && P.fe && P.elasto_on && !P.abc_1D) GF_CU(wait_(st, ev_fe, 0));
         // the mixed form's RK kernel updates two cells per thread
         const unsigned brk = is_mixed<R>::value ? blocks_for(P.n, 2 * kThreads) : bn;
         GF_CU(klaunch(eng, "k_elastic_rk", k_elastic_rk<S, R>, dim3(brk), dim3(kThreads), 0, st, P, io));

@@ -270,6 +270,21 @@ def test_magnetic_materials_that_no_cell_has(gf, precision):
     _same(got, want, TOL[precision])
 
 
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("shape", [(6, 12, 10), (64, 64, 32)])
+def test_liao_boundary_waits_for_the_strain_of_the_first_stage(gf, shape, precision):
+    """The first step from an uploaded u, whose k = 0 plane the boundary replaces:
+    the branches of a stage give what its kernels give one after another."""
+    d = _moving(_fe(gf, *shape, abc_1D=False), 67)
+    out = []
+    for profiled in (False, True):
+        with gf.Engine.from_params(d, device=0, precision=precision) as e:
+            e.profile_steps(2) if profiled else e.advance(2)
+            out.append([e.download(f) for f in ("p", "q", "u", "v", "Ex")])
+    for x, y in zip(*out):
+        assert np.array_equal(x, y)
+
+
 def test_opposite_sublattices_have_no_moment(gf):
     D = gf.decks
     d = D.preset_fm_demag(nx=6, ny=5, nz=4, steps=5)
